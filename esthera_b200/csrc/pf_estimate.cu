@@ -1,8 +1,9 @@
 // pf_estimate.cu -- posterior estimate of a set of particles as a kernel-level
-// entry point: per-sub-filter FP64 partials (one CTA each) into a scratch
-// array in global memory, then one CTA combining them with log-sum-exp
-// rescaling.  The same arithmetic as the filter's own estimate: weights
-// exp(key - max) in FP32, sums in FP64, circular means for angular variables,
+// entry point: FP64 partial sums of the sub-filters into a scratch array in
+// global memory (k_est_partials, a warp or a CTA per sub-filter, one row per
+// CTA), then one CTA combining the rows with log-sum-exp rescaling.  The same
+// arithmetic as the filter's own estimate: weights exp(key - max) in FP32 with
+// the sub-filter's maximum, sums in FP64, circular means for angular variables,
 // the reference's winner (first maximum key, thrust::max_element semantics,
 // src/partfilt/cuda/pf_generic_soa.cu:1014-1017).
 #include <cstring>
@@ -16,183 +17,325 @@
 namespace pfdev {
 
 constexpr int kEstMaxState = 16;
-constexpr int kEstStride = 3 + 2 * kEstMaxState;  // doubles per sub-filter: lmax, W, sums[S], cos[S], best
+// A row of partials: [0] key maximum (0 in linear mode), [1] the first-maximum
+// winner's key, [2] its particle index (-1: every key is NaN), [3] sum w,
+// [4+v] sum w x_v (angles: sum w sin x_v), [4+S+a] sum w cos of the a-th angle.
+constexpr int kEstStride = 4 + 2 * kEstMaxState;
+constexpr int kEstFinalThreads = 512;
 
-// Partials of sub-filter blockIdx.x: [0] key max (0 in linear mode), [1] sum w,
-// [2+v] sum w x_v (angles: sum w sin x_v), [2+S+v] sum w cos x_v, [2+2S] index of
-// the first maximal key within the sub-filter.
-__global__ void __launch_bounds__(256) k_est_partials(const float* __restrict__ keys, const float* __restrict__ state,
-                                                      int S, int64_t T, int m, uint32_t angle_mask, int log_weights,
-                                                      double* __restrict__ part)
+// V consecutive floats (V = 4: one 16-byte load).
+template <int V>
+__device__ __forceinline__ void est_load(const float* __restrict__ p, float (&o)[V])
 {
-    __shared__ double red[8][kEstStride];
-    __shared__ float rk[8];
-    __shared__ int ri[8];
-    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    const int64_t base = (int64_t)b * m;
-    float bk = -INFINITY;
-    int bi = 0x7fffffff;
-    for (int i = tid; i < m; i += 256) {
-        const float k = keys[base + i];
-        if (k > bk || (k == bk && i < bi)) {
-            bk = k;
-            bi = i;
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ok = __shfl_xor_sync(kFull, bk, o);
-        const int oi = __shfl_xor_sync(kFull, bi, o);
-        if (ok > bk || (ok == bk && oi < bi)) {
-            bk = ok;
-            bi = oi;
-        }
-    }
-    if (lane == 0) {
-        rk[wp] = bk;
-        ri[wp] = bi;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        for (int w = 1; w < 8; ++w)
-            if (rk[w] > rk[0] || (rk[w] == rk[0] && ri[w] < ri[0])) {
-                rk[0] = rk[w];
-                ri[0] = ri[w];
-            }
-    }
-    __syncthreads();
-    const float lmax = log_weights ? rk[0] : 0.0f;
-    double acc[kEstStride - 1];
-#pragma unroll
-    for (int j = 0; j < kEstStride - 1; ++j) acc[j] = 0.0;
-    for (int i = tid; i < m; i += 256) {
-        const float k = keys[base + i];
-        const double w = log_weights ? (double)__expf(k - lmax) : (double)k;
-        acc[0] += w;
-#pragma unroll
-        for (int v = 0; v < kEstMaxState; ++v) {
-            if (v < S) {
-                const float x = state[(int64_t)v * T + base + i];
-                if ((angle_mask >> v) & 1u) {
-                    float sn, cs;
-                    __sincosf(x, &sn, &cs);
-                    acc[1 + v] += w * (double)sn;
-                    acc[1 + kEstMaxState + v] += w * (double)cs;
-                } else {
-                    acc[1 + v] += w * (double)x;
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < kEstStride - 1; ++j) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(kFull, acc[j], o);
-        if (lane == 0) red[wp][j] = acc[j];
-    }
-    __syncthreads();
-    double* out = part + (int64_t)b * kEstStride;
-    for (int j = tid; j < kEstStride - 1; j += 256) {
-        double s = red[0][j];
-        for (int w = 1; w < 8; ++w) s += red[w][j];
-        // [0] lmax, [1] W, [2..] sums (compacted: sin/linear at 2+v, cos at 2+S+v)
-        if (j == 0) out[1] = s;
-        else if (j <= kEstMaxState) {
-            if (j - 1 < S) out[2 + (j - 1)] = s;
-        } else if (j - 1 - kEstMaxState < S) {
-            out[2 + S + (j - 1 - kEstMaxState)] = s;
-        }
-    }
-    if (tid == 0) {
-        out[0] = (double)lmax;
-        out[2 + 2 * S] = (double)ri[0];
+    if constexpr (V == 4) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+        o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+    } else {
+        o[0] = __ldg(p);
     }
 }
 
-// Combine nsub partials into one pf_estimate (one CTA of 256 threads).
-__global__ void __launch_bounds__(256) k_est_final(const double* __restrict__ part, const float* __restrict__ keys,
-                                                   const float* __restrict__ state, int S, int64_t T, int m,
-                                                   int nsub, uint32_t angle_mask, int log_weights,
-                                                   pf_estimate* __restrict__ out)
+// Partial sums of the sub-filters, TW warps each (TW = 1: the CTA's four warps
+// take four sub-filters; TW = 8: the CTA's eight warps share one), combined in
+// shared memory into one row per CTA.  V = 4 reads four particles a lane and
+// load, for rows that are 16-byte aligned.
+//
+// Bound: reading 4 (1 + S) bytes per particle.  The first R loads of the keys
+// -- and, for states of up to 4 variables, of every state row -- are issued
+// before the maximum is reduced, so a sub-filter costs one round trip to
+// memory, and a lane keeps its own sums only for the variables there are.  2^20
+// particles of 3 variables, 2048 sub-filters of 512: 10.6 us (cold) against 59.0 us for one
+// 256-thread CTA per sub-filter with 33 sums per thread whatever S was.
+template <int S, int TW, int V>
+__global__ void __launch_bounds__(TW == 1 ? 128 : 256)
+    k_est_partials(const float* __restrict__ keys, const float* __restrict__ state, int64_t T, int m, int nsub,
+                   uint32_t angle_mask, int log_weights, double* __restrict__ part)
 {
-    __shared__ double red[8][kEstStride];
-    __shared__ float rk[8];
-    __shared__ int64_t rg[8];
-    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    double gmax = -INFINITY;
-    float bk = -INFINITY;
-    int64_t bg = INT64_MAX;
-    for (int b = tid; b < nsub; b += 256) {
-        const double* p = part + (int64_t)b * kEstStride;
-        gmax = fmax(gmax, p[0]);
-        const int64_t g = (int64_t)b * m + (int64_t)p[2 + 2 * S];
-        const float k = keys[g];
-        if (k > bk || (k == bk && g < bg)) {
-            bk = k;
-            bg = g;
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        gmax = fmax(gmax, __shfl_xor_sync(kFull, gmax, o));
-        const float ok = __shfl_xor_sync(kFull, bk, o);
-        const int64_t og = __shfl_xor_sync(kFull, bg, o);
-        if (ok > bk || (ok == bk && og < bg)) {
-            bk = ok;
-            bg = og;
-        }
-    }
-    if (lane == 0) {
-        red[wp][0] = gmax;
-        rk[wp] = bk;
-        rg[wp] = bg;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        for (int w = 1; w < 8; ++w) {
-            red[0][0] = fmax(red[0][0], red[w][0]);
-            if (rk[w] > rk[0] || (rk[w] == rk[0] && rg[w] < rg[0])) {
-                rk[0] = rk[w];
-                rg[0] = rg[w];
+    constexpr int NW = TW == 1 ? 4 : 8;          // warps in the CTA
+    constexpr int R = V == 4 ? 4 : 8;            // loads of the keys held in registers
+    constexpr bool PRE = S <= 4 && V == 4;       // and of the state rows
+    __shared__ double red[NW][kEstStride];
+    allow_dependents();
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int wt = wp % TW;                      // warp within the sub-filter's team
+    const int b = blockIdx.x * (NW / TW) + wp / TW;
+    const bool on = b < nsub;                    // the same for a whole team
+    const int64_t base = (int64_t)b * m;
+    const unsigned n = (unsigned)m, i0 = on ? (unsigned)((wt * 32 + lane) * V) : n;
+    constexpr unsigned step = TW * 32 * V;
+    float k[R][V], x[PRE ? R : 1][S][V];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const unsigned i = i0 + r * step;
+        if (i < n) {
+            est_load<V>(keys + base + i, k[r]);
+            if constexpr (PRE) {
+#pragma unroll
+                for (int v = 0; v < S; ++v) est_load<V>(state + v * T + base + i, x[r][v]);
             }
         }
     }
-    __syncthreads();
-    const double gm = log_weights ? red[0][0] : 0.0;
-    const int64_t best = (rg[0] >= 0 && rg[0] < T) ? rg[0] : 0;
-    __syncthreads();
-    const int nv = 1 + 2 * S;
-    double acc[1 + 2 * kEstMaxState];
+    // the maximum and the first particle that holds it (a NaN key never does)
+    float bk = -INFINITY;
+    int bi = 0x7fffffff;
+    auto offer = [&](float key, int i) {
+        if (key > bk || (key == bk && i < bi)) {
+            bk = key;
+            bi = i;
+        }
+    };
 #pragma unroll
-    for (int j = 0; j < 1 + 2 * kEstMaxState; ++j) acc[j] = 0.0;
-    for (int b = tid; b < nsub; b += 256) {
-        const double* p = part + (int64_t)b * kEstStride;
-        const double sc = log_weights ? exp(p[0] - gm) : 1.0;
+    for (int r = 0; r < R; ++r) {
+        const unsigned i = i0 + r * step;
+        if (i < n) {
 #pragma unroll
-        for (int j = 0; j < 1 + 2 * kEstMaxState; ++j)
-            if (j < nv) acc[j] += sc * p[1 + j];
+            for (int q = 0; q < V; ++q) offer(k[r][q], (int)i + q);
+        }
+    }
+    for (unsigned i = i0 + R * step; i < n; i += step) {
+        float kk[V];
+        est_load<V>(keys + base + i, kk);
+#pragma unroll
+        for (int q = 0; q < V; ++q) offer(kk[q], (int)i + q);
     }
 #pragma unroll
-    for (int j = 0; j < 1 + 2 * kEstMaxState; ++j) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ok = __shfl_xor_sync(kFull, bk, o);
+        const int oi = __shfl_xor_sync(kFull, bi, o);
+        offer(ok, oi);
+    }
+    if constexpr (TW > 1) {
+        __shared__ float rk[NW];
+        __shared__ int ri[NW];
+        if (lane == 0) {
+            rk[wp] = bk;
+            ri[wp] = bi;
+        }
+        __syncthreads();
+        for (int w = 0; w < NW; ++w) offer(rk[w], ri[w]);
+    }
+    const float lmax = log_weights ? bk : 0.0f;
+    double sw = 0.0, ss[S], sc[S];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(kFull, acc[j], o);
-        if (lane == 0) red[wp][j] = acc[j];
+    for (int v = 0; v < S; ++v) ss[v] = sc[v] = 0.0;
+    auto add = [&](const float (&kk)[V], auto&& row) {
+        double w[V];
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+            w[q] = log_weights ? (double)__expf(kk[q] - lmax) : (double)kk[q];
+            sw += w[q];
+        }
+#pragma unroll
+        for (int v = 0; v < S; ++v) {
+            float xv[V];
+            row(v, xv);
+            if ((angle_mask >> v) & 1u) {
+#pragma unroll
+                for (int q = 0; q < V; ++q) {
+                    float sn, cs;
+                    __sincosf(xv[q], &sn, &cs);
+                    ss[v] = fma(w[q], (double)sn, ss[v]);
+                    sc[v] = fma(w[q], (double)cs, sc[v]);
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < V; ++q) ss[v] = fma(w[q], (double)xv[q], ss[v]);
+            }
+        }
+    };
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const unsigned i = i0 + r * step;
+        if (i < n) {
+            add(k[r], [&](int v, float(&o)[V]) {
+                if constexpr (PRE) {
+#pragma unroll
+                    for (int q = 0; q < V; ++q) o[q] = x[r][v][q];
+                } else {
+                    est_load<V>(state + v * T + base + i, o);
+                }
+            });
+        }
+    }
+    for (unsigned i = i0 + R * step; i < n; i += step) {
+        float kk[V];
+        est_load<V>(keys + base + i, kk);
+        add(kk, [&](int v, float(&o)[V]) { est_load<V>(state + v * T + base + i, o); });
+    }
+    auto tree = [&](double a) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(kFull, a, o);
+        return a;
+    };
+    sw = tree(sw);
+    if (lane == 0) {
+        red[wp][0] = on ? (double)lmax : -INFINITY;
+        red[wp][1] = (double)bk;
+        red[wp][2] = on && bi < m ? (double)(base + bi) : -1.0;
+        red[wp][3] = sw;
+    }
+    int a = 0;
+#pragma unroll
+    for (int v = 0; v < S; ++v) {
+        const double s = tree(ss[v]);
+        if (lane == 0) red[wp][4 + v] = s;
+        if ((angle_mask >> v) & 1u) {
+            const double c = tree(sc[v]);
+            if (lane == 0) red[wp][4 + S + a] = c;
+            ++a;
+        }
     }
     __syncthreads();
-    if (tid == 0) {
-        for (int w = 1; w < 8; ++w)
-            for (int j = 0; j < nv; ++j) red[0][j] += red[w][j];
-        const double W = red[0][0];
-        pf_estimate e;
-        memset(&e, 0, sizeof(e));
-        for (int v = 0; v < S; ++v)
-            e.mean[v] = ((angle_mask >> v) & 1u) ? atan2(red[0][1 + v], red[0][1 + S + v]) : red[0][1 + v] / W;
-        e.log_norm = gm + log(W);
-        for (int v = 0; v < S; ++v) e.best[v] = state[(int64_t)v * T + best];
-        e.best_key = keys[best];
-        e.best_subfilter = (int32_t)(best / m);
-        e.step = 0;
-        e.flags = (isfinite(gm) && isfinite(W) && W > 0.0) ? 0 : 1;
-        *out = e;
+    // one row: the warps' sums scaled to the CTA's maximum (a team's warps have the same one)
+    double* out = part + (int64_t)blockIdx.x * kEstStride;
+    const int nw = min(NW, (nsub - (int)blockIdx.x * (NW / TW)) * TW);  // warps that had a sub-filter
+    double cm = red[0][0];
+    for (int w = 1; w < nw; ++w) cm = fmax(cm, red[w][0]);
+    for (int j = 3 + threadIdx.x; j < 4 + S + a; j += blockDim.x) {
+        double s = 0.0;
+        for (int w = 0; w < nw; ++w) {
+            const double l = red[w][0];
+            s += (log_weights && l != cm ? exp(l - cm) : 1.0) * red[w][j];
+        }
+        out[j] = s;
     }
+    if (threadIdx.x == 0) {
+        double wk = -INFINITY, wi = -1.0;
+        for (int w = 0; w < nw; ++w) {
+            const double ok = red[w][1], oi = red[w][2];
+            if (oi >= 0.0 && (wi < 0.0 || ok > wk || (ok == wk && oi < wi))) {
+                wk = ok;
+                wi = oi;
+            }
+        }
+        out[0] = cm;
+        out[1] = wk;
+        out[2] = wi;
+    }
+}
+
+// Combine the rows into one pf_estimate (one CTA; a programmatic dependent of
+// k_est_partials).  Bound: two round trips to L2 and the exponentials between
+// them.  Thread r weighs row r, then each warp adds every 16th row, lane j its
+// value j (a row is one coalesced read), in windows of 512 rows.  512 rows: 13.2 us (cold)
+// against 18.4 us for one thread per row holding all 33 sums.
+__global__ void __launch_bounds__(kEstFinalThreads)
+    k_est_final(const double* __restrict__ part, const float* __restrict__ keys, const float* __restrict__ state,
+                int S, int64_t T, int m, int nrow, uint32_t angle_mask, int log_weights, pf_estimate* __restrict__ out)
+{
+    constexpr int NW = kEstFinalThreads / 32;
+    __shared__ double red[NW][kEstStride];
+    __shared__ double scale[kEstFinalThreads];
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    wait_prerequisites();
+    double gm = -INFINITY, bk = -INFINITY, bi = -1.0;
+    auto offer = [&](double ok, double oi) {
+        if (oi >= 0.0 && (bi < 0.0 || ok > bk || (ok == bk && oi < bi))) {
+            bk = ok;
+            bi = oi;
+        }
+    };
+    for (int r = tid; r < nrow; r += kEstFinalThreads) {
+        const double* p = part + (int64_t)r * kEstStride;
+        gm = fmax(gm, __ldcg(p));
+        offer(__ldcg(p + 1), __ldcg(p + 2));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        gm = fmax(gm, __shfl_xor_sync(kFull, gm, o));
+        const double ok = __shfl_xor_sync(kFull, bk, o);
+        const double oi = __shfl_xor_sync(kFull, bi, o);
+        offer(ok, oi);
+    }
+    if (lane == 0) {
+        red[wp][0] = gm;
+        red[wp][1] = bk;
+        red[wp][2] = bi;
+    }
+    __syncthreads();
+    for (int w = 0; w < NW; ++w) {
+        gm = fmax(gm, red[w][0]);
+        offer(red[w][1], red[w][2]);
+    }
+    if (!log_weights) gm = 0.0;
+    const int nv = 1 + S + __popc(angle_mask & ((1u << S) - 1u));
+    double a0 = 0.0, a1 = 0.0;  // values lane and lane + 32
+    for (int r0 = 0; r0 < nrow; r0 += kEstFinalThreads) {
+        const int nr = min(kEstFinalThreads, nrow - r0);
+        __syncthreads();
+        if (tid < nr) scale[tid] = log_weights ? exp(__ldcg(part + (int64_t)(r0 + tid) * kEstStride) - gm) : 1.0;
+        __syncthreads();
+        const double* p = part + (int64_t)r0 * kEstStride + 3 + lane;
+        if (lane < nv) {
+#pragma unroll 8
+            for (int r = wp; r < nr; r += NW) a0 += scale[r] * __ldcg(p + (int64_t)r * kEstStride);
+        }
+        if (lane + 32 < nv)
+            for (int r = wp; r < nr; r += NW) a1 += scale[r] * __ldcg(p + 32 + (int64_t)r * kEstStride);
+    }
+    __syncthreads();
+    red[wp][lane] = a0;
+    if (lane + 32 < nv) red[wp][lane + 32] = a1;
+    __syncthreads();
+    if (wp != 0) return;
+    __shared__ double sum[kEstStride];
+    for (int j = lane; j < nv; j += 32) {
+        double s = red[0][j];
+        for (int w = 1; w < NW; ++w) s += red[w][j];
+        sum[j] = s;
+    }
+    __syncwarp();
+    const double W = sum[0];
+    const int64_t best = bi >= 0.0 && (int64_t)bi < T ? (int64_t)bi : 0;
+    if (lane < kEstMaxState) {
+        const int v = lane;
+        double mean = 0.0;
+        float bv = 0.0f;
+        if (v < S) {
+            if ((angle_mask >> v) & 1u) {
+                const int c = __popc(angle_mask & ((1u << v) - 1u));
+                mean = atan2(sum[1 + v], sum[1 + S + c]);
+            } else {
+                mean = sum[1 + v] / W;
+            }
+            bv = state[(int64_t)v * T + best];
+        }
+        out->mean[v] = mean;
+        out->best[v] = bv;
+    }
+    if (lane == 0) {
+        out->log_norm = gm + log(W);
+        out->best_key = keys[best];
+        out->best_subfilter = (int32_t)(best / m);
+        out->step = 0;
+        out->flags = (isfinite(gm) && isfinite(W) && W > 0.0) ? 0 : 1;
+    }
+}
+
+// A CTA of eight warps per sub-filter where there are too few sub-filters to
+// fill the GPU with one warp each (four to an SM: 592), or where a sub-filter is
+// longer than two rounds of a warp's loads.
+static bool est_team(int m, int64_t nsub) { return m > 1024 || nsub < 592; }
+static int64_t est_rows(int m, int64_t nsub) { return est_team(m, nsub) ? nsub : (nsub + 3) / 4; }
+
+template <int S>
+static cudaError_t launch_est_partials(const float* keys, const float* state, int64_t T, int m, int nsub,
+                                       uint32_t angle_mask, int log_weights, double* scratch, cudaStream_t st)
+{
+    const bool vec = ((reinterpret_cast<uintptr_t>(keys) | reinterpret_cast<uintptr_t>(state)) & 15) == 0 &&
+                     m % 4 == 0 && T % 4 == 0;
+    const int rows = (int)est_rows(m, nsub);
+#define PF_EST(TW, V) \
+    k_est_partials<S, TW, V><<<rows, TW == 1 ? 128 : 256, 0, st>>>(keys, state, T, m, nsub, angle_mask, log_weights, scratch)
+    if (est_team(m, nsub)) {
+        if (vec) PF_EST(8, 4);
+        else PF_EST(8, 1);
+    } else {
+        if (vec) PF_EST(1, 4);
+        else PF_EST(1, 1);
+    }
+#undef PF_EST
+    return cudaGetLastError();
 }
 
 // Validates the shape and launches partials + final on `st` with the given scratch.
@@ -201,11 +344,26 @@ static cudaError_t launch_estimate(const float* keys, const float* state, int S,
                                    cudaStream_t st)
 {
     const int nsub = (int)(T / m);
-    k_est_partials<<<nsub, 256, 0, st>>>(keys, state, S, T, m, angle_mask, log_weights, scratch);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = cudaErrorInvalidValue;
+    switch (S) {
+#define PF_EST_S(s) \
+    case s: e = launch_est_partials<s>(keys, state, T, m, nsub, angle_mask, log_weights, scratch, st); break;
+        PF_EST_S(1) PF_EST_S(2) PF_EST_S(3) PF_EST_S(4) PF_EST_S(5) PF_EST_S(6) PF_EST_S(7) PF_EST_S(8)
+        PF_EST_S(9) PF_EST_S(10) PF_EST_S(11) PF_EST_S(12) PF_EST_S(13) PF_EST_S(14) PF_EST_S(15) PF_EST_S(16)
+#undef PF_EST_S
+    }
     if (e != cudaSuccess) return e;
-    k_est_final<<<1, 256, 0, st>>>(scratch, keys, state, S, T, m, nsub, angle_mask, log_weights, out);
-    return cudaGetLastError();
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(1);
+    lc.blockDim = dim3(kEstFinalThreads);
+    lc.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, k_est_final, (const double*)scratch, keys, state, S, T, m,
+                              (int)est_rows(m, nsub), angle_mask, log_weights, out);
 }
 
 static bool estimate_shape_ok(int S, int64_t T, int m, std::string* why)
@@ -250,7 +408,7 @@ extern "C" pf_status pfk_estimate(const float* keys, const float* state, int32_t
     pf_estimate* de = nullptr;
     cudaError_t e = cudaMalloc(&dk, (size_t)T * 4);
     if (e == cudaSuccess) e = cudaMalloc(&ds, (size_t)T * num_state * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&dp, (size_t)nsub * kEstStride * 8);
+    if (e == cudaSuccess) e = cudaMalloc(&dp, (size_t)est_rows(m, nsub) * kEstStride * 8);
     if (e == cudaSuccess) e = cudaMalloc(&de, sizeof(pf_estimate));
     if (e == cudaSuccess) e = cudaMemcpy(dk, keys, (size_t)T * 4, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(ds, state, (size_t)T * num_state * 4, cudaMemcpyHostToDevice);
@@ -276,7 +434,7 @@ extern "C" pf_status pfk_estimate(const float* keys, const float* state, int32_t
 // with its per-sub-filter scratch in the static array below (allocated with
 // the module, held by every GPU that loads the library until exit).
 // ---------------------------------------------------------------------------
-constexpr int kNoAllocMaxSubfilters = 4096;  // 4096 * 35 doubles = 1.15 MB per device
+constexpr int kNoAllocMaxSubfilters = 4096;  // 4096 * 36 doubles = 1.18 MB per device
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocMaxSubfilters * kEstStride];
 
 static std::mutex g_noalloc_mu;
