@@ -61,43 +61,6 @@ __device__ __forceinline__ void mtgp_load(MtgpSmem& s, const uint32_t* __restric
     __syncthreads();
 }
 
-// mtgp_load with the global reads of the stream words issued first (into
-// registers, NT threads) and `work()` run while they are in flight -- the
-// sampling kernels compute the step's model constants there.  Same result as
-// mtgp_load; ends with a barrier.
-template <int NT, class Work>
-__device__ __forceinline__ void mtgp_load_overlap(MtgpSmem& s, const uint32_t* __restrict__ gstate, int set,
-                                                  uint32_t mask, Work work)
-{
-    constexpr int R = (kMtgpN + NT - 1) / NT;
-    const int tid = threadIdx.x;
-    uint32_t w[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int i = tid + r * NT;
-        w[r] = i < kMtgpN ? __ldcs(gstate + i) : 0u;
-    }
-    const uint32_t* P = g_mtgp_params + set * 52;
-    const uint32_t tb = tid < 16 ? P[4 + tid] : 0u, tt = tid < 16 ? P[36 + tid] : 0u;
-    work();
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int i = tid + r * NT;
-        if (i < kMtgpN) s.ring[i] = w[r];
-    }
-    if (tid < 16) {
-        s.tbl[tid] = tb;
-        s.ttb[tid] = tt;
-    }
-    if (tid == 0) {
-        s.pos = P[0];
-        s.sh1 = P[1];
-        s.sh2 = P[2];
-        s.mask = mask ? mask : P[3];
-    }
-    __syncthreads();
-}
-
 // Generate n outputs of the stream held in s.ring, in rounds of 256:
 // output k: x_{k+351} = rec(x_k, x_{k+1}, x_{k+pos}); out_k = temper(x_{k+351}, x_{k+pos-1}).
 // Within a round every read index is < base+351 <= every write index, so
@@ -154,62 +117,130 @@ __device__ __forceinline__ void box_muller(float x, float y, float& z1, float& z
     z2 = -r * s;
 }
 
-// mtgp_generate for float output with the first nbm words (nbm even) turned
-// into normals by Box-Muller on the fly: each thread produces the adjacent
-// words (k, k+1) of a round, so the pair's recursion inputs come in 64-bit
-// shared loads and the normals go out as one 64-bit store to nz[k], nz[k+1]
-// (the same values as mtgp_generate followed by box_muller on nz[2q], nz[2q+1]).
-// Words k >= nbm (k < n) go to emit(k, word).  Ends with a barrier.
-// RAW: the first nbm words are stored as they are (floats in [1,2)) and the
-// caller applies box_muller to each pair (nz[2q], nz[2q+1]) when it reads
-// them; the same normals, with the Box-Muller chains taken out of the
-// barrier-separated rounds.
-template <bool RAW = false, class Emit>
-__device__ __forceinline__ void mtgp_generate_bm(MtgpSmem& s, int n, int nbm, float* __restrict__ nz, Emit emit)
+// The sampling kernels' generator: the stream words of up to CAP outputs in a
+// row in shared memory, word k of the recursion at x[k - shift], so that a
+// thread's addresses advance by a constant per round (a 1024-word ring's masks
+// and base additions were about a third of the round's instructions).  When
+// the next round would not fit, the last 351 words move to the front.
+template <int CAP>
+struct MtgpLinear {
+    uint32_t x[((kMtgpN + 1) + CAP + 3) / 4 * 4];
+    uint32_t tbl[16];
+    uint32_t ttb[16];  // flt_tmp_tbl
+    uint32_t pos, sh1, sh2, mask;
+};
+// Outputs held at once for nbm normals: all of them and the round that
+// finishes the step, at most 2048.
+constexpr int mtgp_cap(int nbm) { return ((nbm + 255) / 256 + 1) * 256 < 2048 ? ((nbm + 255) / 256 + 1) * 256 : 2048; }
+
+// Stream words x_0..x_350 -> x[0..350] and the parameter set's tables, with the
+// global reads issued first (into registers, NT threads) and `work()` run while
+// they are in flight -- the sampling kernel computes the step's model constants
+// there.  Ends with a barrier.
+template <int NT, int CAP, class Work>
+__device__ __forceinline__ void mtgp_load_linear(MtgpLinear<CAP>& s, const uint32_t* __restrict__ gstate, int set,
+                                                 uint32_t mask, Work work)
 {
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const uint32_t pos = s.pos, sh1 = s.sh1, sh2 = s.sh2, mask = s.mask;
-    const uint32_t* ring = s.ring;
-    auto ld2 = [&](int i) { return *reinterpret_cast<const uint2*>(ring + (i & 1023)); };  // i even
+    constexpr int R = (kMtgpN + NT - 1) / NT;
+    const int tid = threadIdx.x;
+    uint32_t w[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = tid + r * NT;
+        w[r] = i < kMtgpN ? __ldcs(gstate + i) : 0u;
+    }
+    const uint32_t* P = g_mtgp_params + set * 52;
+    const uint32_t tb = tid < 16 ? P[4 + tid] : 0u, tt = tid < 16 ? P[36 + tid] : 0u;
+    work();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = tid + r * NT;
+        if (i < kMtgpN) s.x[i] = w[r];
+    }
+    if (tid < 16) {
+        s.tbl[tid] = tb;
+        s.ttb[tid] = tt;
+    }
+    if (tid == 0) {
+        s.pos = P[0];
+        s.sh1 = P[1];
+        s.sh2 = P[2];
+        s.mask = mask ? mask : P[3];
+    }
+    __syncthreads();
+}
+
+// The stream's next n outputs (the recursion and tempering of mtgp_generate,
+// float output), in rounds of 256, each thread producing adjacent words (k,
+// k+1).  The first nbm (even) are turned into normals by Box-Muller into nz[k],
+// nz[k+1] -- RAW: stored as they are (floats in [1,2)) and the caller applies
+// box_muller to each pair (nz[2q], nz[2q+1]) when it reads them: the same
+// normals, with the Box-Muller chains taken out of the barrier-separated
+// rounds.  Words k >= nbm (k < n) go to emit(k, word).  Returns the shift: the
+// stream's next state word i is x[n + i - shift].  Ends with a barrier.
+template <bool RAW, int NT, int CAP, class Emit>
+__device__ __forceinline__ int mtgp_generate_linear(MtgpLinear<CAP>& s, int n, int nbm, float* __restrict__ nz,
+                                                    Emit emit)
+{
+    constexpr int PR = (kMtgpLanes / 2 + NT - 1) / NT;  // pairs per thread and round
+    const int tid = threadIdx.x;
+    const uint32_t sh1 = s.sh1, sh2 = s.sh2, mask = s.mask;
+    const int pos = (int)s.pos;
+    const bool odd = pos & 1;
+    int shift = 0;
+    auto pair = [&](uint32_t* x, uint32_t& o0, uint32_t& o1) {
+        const uint2 x01 = *reinterpret_cast<const uint2*>(x);
+        const uint32_t x2 = x[2];
+        uint32_t t0, y0, y1;
+        if (odd) {
+            const uint2 ty = *reinterpret_cast<const uint2*>(x + pos - 1);
+            t0 = ty.x;
+            y0 = ty.y;
+            y1 = x[pos + 1];
+        } else {
+            const uint2 yy = *reinterpret_cast<const uint2*>(x + pos);
+            t0 = x[pos - 1];
+            y0 = yy.x;
+            y1 = yy.y;
+        }
+        uint32_t xa = (x01.x & mask) ^ x01.y;
+        uint32_t xb = (x01.y & mask) ^ x2;
+        xa ^= xa << sh1;
+        xb ^= xb << sh1;
+        const uint32_t ya = xa ^ (y0 >> sh2);
+        const uint32_t yb = xb ^ (y1 >> sh2);
+        const uint32_t r0 = ya ^ s.tbl[ya & 0x0f];
+        const uint32_t r1 = yb ^ s.tbl[yb & 0x0f];
+        x[kMtgpN] = r0;
+        x[kMtgpN + 1] = r1;
+        uint32_t ta = t0 ^ (t0 >> 16), tb = y0 ^ (y0 >> 16);
+        ta ^= ta >> 8;
+        tb ^= tb >> 8;
+        o0 = (r0 >> 9) ^ s.ttb[ta & 0x0f];
+        o1 = (r1 >> 9) ^ s.ttb[tb & 0x0f];
+    };
     for (int base = 0; base < n; base += kMtgpLanes) {
-        for (int l2 = tid; l2 < kMtgpLanes / 2; l2 += nt) {
-            const int k = base + 2 * l2;  // even
+        if (base - shift + kMtgpLanes > CAP) {  // the same in every thread
+            constexpr int R = (kMtgpN + NT - 1) / NT;
+            uint32_t w[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) w[r] = s.x[min(tid + r * NT, kMtgpN - 1) + base - shift];
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (tid + r * NT < kMtgpN) s.x[tid + r * NT] = w[r];
+            shift = base;
+            __syncthreads();
+        }
+#pragma unroll
+        for (int q = 0; q < PR; ++q) {
+            const int l = 2 * (tid + q * NT), k = base + l;
             // past the requested words (the last round): nothing this pair
             // writes is read again -- the state kept is x_n .. x_{n+350}, the
             // last of which pair (n-2, n-1) writes
-            if (k >= n) continue;
-            const uint2 x01 = ld2(k), x23 = ld2(k + 2);
-            uint32_t t0, y0, y1;
-            if ((pos & 1u) == 0) {
-                const uint2 yy = ld2(k + (int)pos);
-                y0 = yy.x;
-                y1 = yy.y;
-                t0 = ld2(k + (int)pos - 2).y;
-            } else {
-                const uint2 ty = ld2(k + (int)pos - 1), y2 = ld2(k + (int)pos + 1);
-                t0 = ty.x;
-                y0 = ty.y;
-                y1 = y2.x;
-            }
-            const uint32_t t1 = y0;
-            uint32_t xa = (x01.x & mask) ^ x01.y;
-            xa ^= xa << sh1;
-            uint32_t ya = xa ^ (y0 >> sh2);
-            const uint32_t r0 = ya ^ s.tbl[ya & 0x0f];
-            uint32_t xb = (x01.y & mask) ^ x23.x;
-            xb ^= xb << sh1;
-            uint32_t yb = xb ^ (y1 >> sh2);
-            const uint32_t r1 = yb ^ s.tbl[yb & 0x0f];
-            s.ring[(k + kMtgpN) & 1023] = r0;
-            s.ring[(k + kMtgpN + 1) & 1023] = r1;
-            uint32_t ta = t0;
-            ta ^= ta >> 16;
-            ta ^= ta >> 8;
-            uint32_t tb = t1;
-            tb ^= tb >> 16;
-            tb ^= tb >> 8;
-            const uint32_t o0 = (r0 >> 9) ^ s.ttb[ta & 0x0f];
-            const uint32_t o1 = (r1 >> 9) ^ s.ttb[tb & 0x0f];
+            if (l >= kMtgpLanes || k >= n) continue;
+            uint32_t o0, o1;
+            pair(s.x + (k - shift), o0, o1);
             if (k < nbm) {
                 if constexpr (RAW) {
                     *reinterpret_cast<uint2*>(nz + k) = make_uint2(o0, o1);
@@ -219,12 +250,21 @@ __device__ __forceinline__ void mtgp_generate_bm(MtgpSmem& s, int n, int nbm, fl
                     *reinterpret_cast<float2*>(nz + k) = make_float2(z1, z2);
                 }
             } else {
-                if (k < n) emit(k, o0);
+                emit(k, o0);
                 if (k + 1 < n) emit(k + 1, o1);
             }
         }
         __syncthreads();
     }
+    return shift;
+}
+
+// State after n outputs: x_n .. x_{n+350}.
+template <int CAP>
+__device__ __forceinline__ void mtgp_store_linear(const MtgpLinear<CAP>& s, uint32_t* __restrict__ gstate, int n,
+                                                  int shift)
+{
+    for (int i = threadIdx.x; i < kMtgpN; i += blockDim.x) gstate[i] = s.x[n - shift + i];
 }
 
 // atan2 from an odd polynomial for atan on [0, 1] -- degree 15 in a, i.e. 8
@@ -282,6 +322,58 @@ __device__ __forceinline__ float pf_expneg(float x)
 // sqrt(d2) for d2 >= 0 through the SFU reciprocal square root (0 -> 0).
 __device__ __forceinline__ float pf_sqrt(float d2) { return d2 * rsqrtf(fmaxf(d2, 1e-30f)); }
 
+// E consecutive 4-byte values of shared memory at once (p aligned to 4E bytes
+// where E is 2 or a multiple of 4).
+template <class T>
+__device__ __forceinline__ T word_as(int v)
+{
+    if constexpr (std::is_same<T, float>::value) return __int_as_float(v);
+    else return v;
+}
+__device__ __forceinline__ int as_word(float v) { return __float_as_int(v); }
+__device__ __forceinline__ int as_word(int v) { return v; }
+template <int E, class T>
+__device__ __forceinline__ void lds_row(const T* p, T (&o)[E])
+{
+    if constexpr (E % 4 == 0) {
+#pragma unroll
+        for (int q = 0; q < E; q += 4) {
+            const int4 v = *reinterpret_cast<const int4*>(p + q);
+            o[q] = word_as<T>(v.x);
+            o[q + 1] = word_as<T>(v.y);
+            o[q + 2] = word_as<T>(v.z);
+            o[q + 3] = word_as<T>(v.w);
+        }
+    } else if constexpr (E == 2) {
+        const int2 v = *reinterpret_cast<const int2*>(p);
+        o[0] = word_as<T>(v.x);
+        o[1] = word_as<T>(v.y);
+    } else {
+#pragma unroll
+        for (int q = 0; q < E; ++q) o[q] = p[q];
+    }
+}
+template <int E, class T>
+__device__ __forceinline__ void sts_row(T* p, const T (&o)[E])
+{
+    if constexpr (E % 4 == 0) {
+#pragma unroll
+        for (int q = 0; q < E; q += 4)
+            *reinterpret_cast<int4*>(p + q) =
+                make_int4(as_word(o[q]), as_word(o[q + 1]), as_word(o[q + 2]), as_word(o[q + 3]));
+    } else if constexpr (E == 2) {
+        *reinterpret_cast<int2*>(p) = make_int2(as_word(o[0]), as_word(o[1]));
+    } else {
+#pragma unroll
+        for (int q = 0; q < E; ++q) p[q] = o[q];
+    }
+}
+
+// Shared memory of the sorts: sort_key_words floats (M keys; one word of
+// padding per 32 for rank_sort_desc's search), then M indices.
+__host__ __device__ constexpr int sort_key_words(int M) { return M + ((M / 32 + 3) & ~3); }
+__host__ __device__ constexpr size_t sort_bytes(int M) { return (size_t)(sort_key_words(M) + M) * 4; }
+
 // ---------------------------------------------------------------------------
 // Descending bitonic key+index sort of M keys, E consecutive keys per thread
 // (thread t holds positions E*t .. E*t+E-1).  The comparator network is the
@@ -338,19 +430,19 @@ __device__ __forceinline__ void bitonic_sort_desc(float (&k)[E], int (&ix)[E], f
             } else {
                 __syncthreads();
                 if (writer) {
-#pragma unroll
-                    for (int e = 0; e < E; ++e) {
-                        sk[E * tid + e] = k[e];
-                        si[E * tid + e] = ix[e];
-                    }
+                    sts_row<E>(sk + E * tid, k);
+                    sts_row<E>(si + E * tid, ix);
                 }
                 __syncthreads();
+                float oks[E];
+                int ois[E];
+                lds_row<E>(sk + ((E * tid) ^ stride), oks);
+                lds_row<E>(si + ((E * tid) ^ stride), ois);
 #pragma unroll
                 for (int e = 0; e < E; ++e) {
                     const int p = E * tid + e;
-                    const int q = p ^ stride;
-                    const float ok = sk[q];
-                    const int oi = si[q];
+                    const float ok = oks[e];
+                    const int oi = ois[e];
                     const bool ddd = (p & size) != 0;
                     const bool upper = (p & stride) != 0;
                     const float lo = upper ? ok : k[e];
@@ -371,18 +463,26 @@ __device__ __forceinline__ void bitonic_sort_desc(float (&k)[E], int (&ix)[E], f
 // the sorted permutation is unique, so any correct sort gives the network's
 // result; this one runs the network on the keys alone (a shuffle and a min /
 // max per element and stage instead of two shuffles and four selects), then
-// recovers the permutation: each thread finds the sorted position of each of
-// its keys by a binary search over the sorted keys in shared memory and
-// writes its index there.  If any two keys compare equal (ties, +0 / -0,
-// repeated -inf) or a key is NaN, the whole CTA (every thread takes the same
-// branch) sorts the original (key, index) pairs with bitonic_sort_desc, which
-// keeps the reference network's tie order.  Same contract as
-// bitonic_sort_desc for a CTA owning one sub-filter (tid = threadIdx.x);
-// returns true when the CTA fell back to the full network.  TP as for
+// recovers the permutation: each thread finds the sorted position pos[e] of
+// each of its keys by a binary search over the sorted keys in shared memory.
+// If any two keys compare equal (ties, +0 / -0, repeated -inf) or a key is
+// NaN, the whole CTA (every thread takes the same branch) sorts the original
+// (key, index) pairs with bitonic_sort_desc, which keeps the reference
+// network's tie order.  In: k[e] the key of element E*tid+e; out: k[e] the
+// sorted key at position E*tid+e, pos[e] the sorted position of element
+// E*tid+e.  For a CTA owning one sub-filter (tid = threadIdx.x / TP); returns
+// true when the CTA fell back to the full network.  TP as for
 // bitonic_sort_desc (the pair's lanes hold the same keys).
+//
+// The searched keys are padded by a word per 32: the search's levels read
+// strides of 256, 128, .. 2 keys, which without the padding put up to 16
+// lanes on one bank (2.32M of the sampling kernel's 3.95M shared-load
+// wavefronts at 2^20 particles were such conflicts).  Callers scatter their
+// rows to pos[] and read them back in order, which saves the index round trip
+// and two barriers over gathering.
 // ---------------------------------------------------------------------------
 template <int M, int E, int TP = 1>
-__device__ __forceinline__ bool rank_sort_desc(float (&k)[E], int (&ix)[E], float* sk, int* si)
+__device__ __forceinline__ bool rank_sort_desc(float (&k)[E], int (&pos)[E], float* sk, int* si)
 {
     const int tid = threadIdx.x / TP;
     const bool writer = threadIdx.x % TP == 0;
@@ -424,50 +524,59 @@ __device__ __forceinline__ bool rank_sort_desc(float (&k)[E], int (&ix)[E], floa
                 for (int e = 0; e < E; ++e) v[e] = keep_max ? fmaxf(v[e], o[e]) : fminf(v[e], o[e]);
             } else {
                 __syncthreads();
-                if (writer) {
-#pragma unroll
-                    for (int e = 0; e < E; ++e) sk[E * tid + e] = v[e];
-                }
+                if (writer) sts_row<E>(sk + E * tid, v);
                 __syncthreads();
                 const bool keep_max = ((E * tid) & stride) == 0;
+                float o[E];
+                lds_row<E>(sk + ((E * tid) ^ (first ? size - E : stride)), o);
 #pragma unroll
                 for (int e = 0; e < E; ++e) {
-                    const int p = E * tid + e;
-                    const float o = sk[first ? p ^ (size - 1) : p ^ stride];
-                    v[e] = keep_max ? fmaxf(v[e], o) : fminf(v[e], o);
+                    const float ov = o[first ? E - 1 - e : e];
+                    v[e] = keep_max ? fmaxf(v[e], ov) : fminf(v[e], ov);
                 }
             }
         }
     }
+    constexpr auto pad = [](int p) { return p + (p >> 5); };
     __syncthreads();
     if (writer) {
 #pragma unroll
-        for (int e = 0; e < E; ++e) sk[E * tid + e] = v[e];
+        for (int e = 0; e < E; ++e) sk[pad(E * tid + e)] = v[e];
     }
     __syncthreads();
     bool tie = nan;
 #pragma unroll
     for (int e = 0; e + 1 < E; ++e) tie |= v[e] == v[e + 1];
-    if (E * tid + E < M) tie |= v[E - 1] == sk[E * tid + E];
+    if (E * tid + E < M) tie |= v[E - 1] == sk[pad(E * tid + E)];
     if (__syncthreads_or(tie)) {
+        int ix[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) ix[e] = E * tid + e;
         bitonic_sort_desc<M, E, TP>(k, ix, sk, si, tid, writer);
+        __syncthreads();
+        if (writer) {
+#pragma unroll
+            for (int e = 0; e < E; ++e) si[ix[e]] = E * tid + e;
+        }
+        __syncthreads();
+        lds_row<E>(si + E * tid, pos);
         return true;
     }
-    // sorted position of each original key = the number of keys above it
+    // sorted position of each original key = the number of keys above it; q
+    // is the padded position: a step of 32 or more carries its padding along,
+    // the smaller ones stay within a row of 32
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-        int pos = 0;
+        int q = 0;
 #pragma unroll
-        for (int step = M / 2; step > 0; step >>= 1)
-            if (sk[pos + step - 1] > k[e]) pos += step;
-        if (writer) si[pos] = E * tid + e;
+        for (int step = M / 2; step > 0; step >>= 1) {
+            const int up = step >= 32 ? step + step / 32 : step;
+            if (sk[q + pad(step - 1)] > k[e]) q += up;
+        }
+        pos[e] = q - ((q * 993) >> 15);  // q - q / 33 (q < 33 * 993)
     }
-    __syncthreads();
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        k[e] = v[e];
-        ix[e] = si[E * tid + e];
-    }
+    for (int e = 0; e < E; ++e) k[e] = v[e];
     return false;
 }
 
@@ -516,7 +625,7 @@ __device__ __forceinline__ double scan_f64(const float (&w)[E], double (&cum)[E]
     __syncthreads();
     double v = lane < NW ? red[lane] : 0.0;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
+    for (int d = 1; d < NW; d <<= 1) {  // (levels beyond NW change no lane below NW)
         const double o = __shfl_up_sync(kFull, v, d);
         if (lane >= d) v = v + o;
     }
@@ -559,23 +668,43 @@ __device__ __forceinline__ int upper_count(const double* cum, double x)
 // pos(i) = (u0 + i) * step (cum[-1] = -inf; the last input also takes every
 // output with pos(i) >= cum[M-1]).  Each thread finds, for its E inputs
 // j = E*tid+e, the first output at or above cum[j-1] (an estimate from t /
-// step, corrected with the exact pos(i) comparisons), writes its inputs' runs
-// of outputs to sidx[0..M), and reads back its own E outputs.  pos(i) and the
-// comparisons are those of upper_count(cum, pos(i)), so every output selects
-// the same input (pos is non-decreasing in i).  Synchronises the CTA.
+// step, corrected with the exact pos(i) comparisons); the inputs' runs of
+// outputs tile [0, M) in ascending order.  A run is marked where it starts and
+// at each warp's first output inside it (mark[], zeroed by the caller before
+// its last barrier), and every output takes the largest mark at or before it
+// within its warp.  pos(i) and the comparisons are those of upper_count(cum,
+// pos(i)), so every output selects the same input (pos is non-decreasing in
+// i).  Synchronises the CTA.
+//
+// Bound: latency (FP64 conversions and comparisons in a chain per boundary).
+// At m = 512, 4 particles per thread a CTA of a full grid spends 2870 cycles
+// here, against 3840 when each thread wrote its inputs' runs out one by one --
+// a heavy particle's run is hundreds of outputs long -- after an FP64 division.
 template <int M, int E>
 __device__ __forceinline__ void systematic_select(const double (&cum)[E], double prev, float u0f, double step,
-                                                  int* sidx, int (&sel)[E])
+                                                  int* mark, int (&sel)[E])
 {
     const int tid = threadIdx.x;
+    constexpr int W = 32 * E;  // outputs of a warp
     const double u0 = (double)u0f;
-    const double inv = step > 0.0 ? 1.0 / step : 0.0;
+    // 1 / step for the estimates only: a Newton step from the FP32 reciprocal
+    // (about 1e-13) where that neither over- nor underflows
+    const float sf = (float)step;
+    double inv;
+    if (sf > 1e-30f && sf < 1e30f) {
+        inv = (double)__frcp_rn(sf);
+        inv = fma(inv, fma(-step, inv, 1.0), inv);
+    } else {
+        inv = step > 0.0 ? 1.0 / step : 0.0;
+    }
     auto pos = [&](int i) { return (u0 + (double)i) * step; };
     auto first_at_or_above = [&](double t) {  // first i in [0, M] with pos(i) >= t
-        const double est = ceil(t * inv - u0);
-        int i = est >= 0.0 ? (est <= (double)M ? (int)est : M) : 0;
-        while (i > 0 && pos(i - 1) >= t) --i;
-        while (i < M && pos(i) < t) ++i;
+        const double est = fma(t, inv, -u0);
+        int i = est > 0.0 ? (est < (double)M ? __double2int_ru(est) : M) : 0;
+        if ((i > 0 && pos(i - 1) >= t) || (i < M && pos(i) < t)) {  // the estimate is off: rarely
+            while (i > 0 && pos(i - 1) >= t) --i;
+            while (i < M && pos(i) < t) ++i;
+        }
         return i;
     };
     const int j0 = E * tid;
@@ -584,12 +713,29 @@ __device__ __forceinline__ void systematic_select(const double (&cum)[E], double
     for (int e = 0; e < E; ++e) {
         const int j = j0 + e;
         const int hi = j == M - 1 ? M : first_at_or_above(cum[e]);
-        for (int i = lo; i < hi; ++i) sidx[i] = j;
+        if (lo < hi) {
+            mark[lo] = j;
+            for (int i = (lo / W + 1) * W; i < hi; i += W) mark[i] = j;
+        }
         lo = hi > lo ? hi : lo;
     }
     __syncthreads();
 #pragma unroll
-    for (int e = 0; e < E; ++e) sel[e] = sidx[E * tid + e];
+    for (int e = 0; e < E; ++e) sel[e] = mark[E * tid + e];
+#pragma unroll
+    for (int e = 1; e < E; ++e) sel[e] = max(sel[e], sel[e - 1]);
+    // the largest mark of the lanes before this one
+    int m = sel[E - 1];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(kFull, m, d);
+        if ((tid & 31) >= d) m = max(m, o);
+    }
+    m = __shfl_up_sync(kFull, m, 1);
+    if ((tid & 31) != 0) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) sel[e] = max(sel[e], m);
+    }
 }
 
 // FP32 Blelloch exclusive scan of M values in place (prefix_sum,
@@ -1596,14 +1742,58 @@ struct RareTies<Unicycle> : std::true_type {};
 template <>
 struct RareTies<Beacon> : std::true_type {};
 
-// The sampling kernels' sort of one sub-filter per CTA (see rank_sort_desc).
-template <class Mdl, int M, int E, int TP = 1>
-__device__ __forceinline__ void sort_subfilter(float (&k)[E], int (&ix)[E], float* sk, int* si)
+// The sampling kernels' sort of one sub-filter per CTA: k[e] in, the sorted key
+// at position E*tid+e out, and the particles' state rows in sorted order into
+// stage[v * M + ..], which must be free (nothing reads it once every thread has
+// entered).  Rare ties: every particle is scattered to its sorted position
+// (rank_sort_desc); otherwise the network's indices gather.  store(v, row) gets
+// this thread's E values of sorted row v (a pair's lanes take alternate rows);
+// sorted() runs once the keys are in order.  stage may be read by others until
+// the caller's next barrier.
+template <class Mdl, int M, int E, int TP, class Sorted, class Store>
+__device__ __forceinline__ void sort_subfilter(float (&k)[E], const float (&st)[E][Mdl::S], float* sk, int* si,
+                                               float* stage, Sorted sorted, Store store)
 {
+    constexpr int S = Mdl::S;
+    const int tid = threadIdx.x / TP, h = threadIdx.x % TP;
+    int ix[E];
     if constexpr (RareTies<Mdl>::value) {
         rank_sort_desc<M, E, TP>(k, ix, sk, si);
+        sorted();
+#pragma unroll
+        for (int v = 0; v < S; ++v) {
+            if (v % TP != h) continue;
+#pragma unroll
+            for (int e = 0; e < E; ++e) stage[v * M + ix[e]] = st[e][v];
+        }
     } else {
-        bitonic_sort_desc<M, E, TP>(k, ix, sk, si, threadIdx.x / TP, threadIdx.x % TP == 0);
+#pragma unroll
+        for (int e = 0; e < E; ++e) ix[e] = E * tid + e;
+        bitonic_sort_desc<M, E, TP>(k, ix, sk, si, tid, h == 0);
+        sorted();
+        __syncthreads();  // (a sub-filter of one warp has met no barrier since its normals were read)
+        if (h == 0) {
+#pragma unroll
+            for (int v = 0; v < S; ++v) {
+                float o[E];
+#pragma unroll
+                for (int e = 0; e < E; ++e) o[e] = st[e][v];
+                sts_row<E>(stage + v * M + E * tid, o);
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < S; ++v) {
+        if (v % TP != h) continue;
+        float o[E];
+        if constexpr (RareTies<Mdl>::value) {
+            lds_row<E>(stage + v * M + E * tid, o);
+        } else {
+#pragma unroll
+            for (int e = 0; e < E; ++e) o[e] = stage[v * M + ix[e]];
+        }
+        store(v, o);
     }
 }
 

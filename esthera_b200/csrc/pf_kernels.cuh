@@ -233,17 +233,18 @@ template <class Mdl, int M, int E>
 __device__ __forceinline__ void normals_from_raw(const float* nz, int tid, float (&z)[E][Mdl::K])
 {
 #pragma unroll
-    for (int v = 0; v < Mdl::K; ++v)
+    for (int v = 0; v < Mdl::K; ++v) {
+        float u[E];
+        lds_row<E>(nz + v * M + E * tid, u);
 #pragma unroll
-        for (int e = 0; e < E; e += 2) {
-            const float2 u = *reinterpret_cast<const float2*>(nz + v * M + E * tid + e);
-            box_muller(u.x, u.y, z[e][v], z[e + 1][v]);
-        }
+        for (int e = 0; e < E; e += 2) box_muller(u[e], u[e + 1], z[e][v], z[e + 1][v]);
+    }
 }
 
-// k_sample_sort's dynamic shared memory: the MTGP32 ring (FR), one region
-// holding in turn the normals, the state stage of the sorted gather and the
-// estimate partials' per-thread sums, then the sort keys + indices.
+// k_sample_sort's dynamic shared memory: one region holding in turn the
+// normals, the sorted state rows and the estimate partials' per-thread sums,
+// then one holding the MTGP32 words (FR) and after them the sort's keys and
+// indices.
 template <class Mdl, int M, bool FR, int TP = 1>
 constexpr size_t k1_stage_bytes()
 {
@@ -252,10 +253,13 @@ constexpr size_t k1_stage_bytes()
     if (TP > 1 && stage < (size_t)TP * M * 8) stage = (size_t)TP * M * 8;  // a row of partials per thread
     return nz > stage ? nz : stage;
 }
+template <class Mdl, int M>
+using K1Mtgp = MtgpLinear<mtgp_cap(2 * ((Mdl::K * M + 1) / 2))>;
 template <class Mdl, int M, bool FR, int TP = 1>
 constexpr size_t k1_smem()
 {
-    return (FR ? sizeof(MtgpSmem) : 0) + k1_stage_bytes<Mdl, M, FR, TP>() + (size_t)M * 8;
+    const size_t gen = FR ? sizeof(K1Mtgp<Mdl, M>) : 0;
+    return k1_stage_bytes<Mdl, M, FR, TP>() + (gen > sort_bytes(M) ? gen : sort_bytes(M));
 }
 
 // Estimate partials of one sub-filter from particles in any order:
@@ -358,29 +362,24 @@ __global__ void __launch_bounds__(TP * M / E, pf_min_blocks(TP * M / E, pf_k1_wa
     const int64_t T = D.T;
     const int64_t base = (int64_t)b * M + E * vt;
 
-    unsigned char* p = smem;
-    MtgpSmem* ms = nullptr;
-    if constexpr (FR) {
-        ms = reinterpret_cast<MtgpSmem*>(p);
-        p += sizeof(MtgpSmem);
-    }
-    float* nz = reinterpret_cast<float*>(p);     // normals (FR), later the state stage, then the partials
+    float* nz = reinterpret_cast<float*>(smem);  // normals (FR), later the sorted rows, then the partials
     float* stage = nz;
-    p += k1_stage_bytes<Mdl, M, FR, TP>();
-    float* sk = reinterpret_cast<float*>(p);
-    int* si = reinterpret_cast<int*>(p + (size_t)M * 4);
+    unsigned char* p = smem + k1_stage_bytes<Mdl, M, FR, TP>();
+    float* sk = reinterpret_cast<float*>(p);     // the sort's buffers, over the generator's words
+    int* si = reinterpret_cast<int*>(sk + sort_key_words(M));
 
     if constexpr (FR) {
+        auto& ms = *reinterpret_cast<K1Mtgp<Mdl, M>*>(p);
         uint32_t* gst = D.mtgp + (int64_t)b * kMtgpN;
         // the step's model constants (one warp) while the stream words are in flight
-        mtgp_load_overlap<NT>(*ms, gst, (D.stream_base + b) % kMtgpSets, D.mask, [&] {
+        mtgp_load_linear<NT>(ms, gst, (D.stream_base + b) % kMtgpSets, D.mask, [&] {
             if (tid < 32) Mdl::prepare(cst, *input_of(in, f), D.mp, tid);
         });
         const int nbm = D.nbm;
         float* ru = D.ru + (int64_t)b * D.ru_stride;
-        mtgp_generate_bm<raw_normals<Mdl, E>()>(*ms, D.draws, nbm, nz,
-                                                [&](int k, uint32_t o) { ru[k - nbm] = __uint_as_float(o); });
-        mtgp_store(*ms, gst, D.draws);
+        const int shift = mtgp_generate_linear<raw_normals<Mdl, E>(), NT>(
+            ms, D.draws, nbm, nz, [&](int k, uint32_t o) { ru[k - nbm] = __uint_as_float(o); });
+        mtgp_store_linear(ms, gst, D.draws, shift);
     } else {
         if (tid < 32) Mdl::prepare(cst, *input_of(in, f), D.mp, tid);
     }
@@ -420,34 +419,18 @@ __global__ void __launch_bounds__(TP * M / E, pf_min_blocks(TP * M / E, pf_k1_wa
         }
     }
     float k[E];
-    int ix[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        k[e] = okey[e];
-        ix[e] = E * vt + e;
-    }
-    sort_subfilter<Mdl, M, E, TP>(k, ix, sk, si);
-    if (writer) stv<E>(D.tkey + base, k);
-    __syncthreads();  // normals consumed, sort buffers free: stage the state
-    if (writer) {
-#pragma unroll
-        for (int v = 0; v < S; ++v)
-#pragma unroll
-            for (int e = 0; e < E; ++e) stage[v * M + E * vt + e] = st[e][v];
-    }
-    if (tid == 0) {
-        D.winner[b] = k[0];
-        s_lmax = k[0];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < S; ++v) {
-        if (v % TP != h) continue;  // a pair's lanes gather alternate variables
-        float o[E];
-#pragma unroll
-        for (int e = 0; e < E; ++e) o[e] = stage[v * M + ix[e]];
-        stv<E>(D.tmp + v * T + base, o);
-    }
+    for (int e = 0; e < E; ++e) k[e] = okey[e];
+    sort_subfilter<Mdl, M, E, TP>(
+        k, st, sk, si, stage,
+        [&] {
+            if (writer) stv<E>(D.tkey + base, k);
+            if (tid == 0) {
+                D.winner[b] = k[0];
+                s_lmax = k[0];
+            }
+        },
+        [&](int v, const float(&o)[E]) { stv<E>(D.tmp + v * T + base, o); });
     write_partials<Mdl, E, NT, k1_stage_bytes<Mdl, M, FR, TP>()>(D, b, D.log_weights ? s_lmax : 0.0f, okey, st, sn,
                                                                   cs, reinterpret_cast<double*>(stage), writer);
 }
@@ -1041,7 +1024,7 @@ template <int S, int M, int E, int RES>
 constexpr size_t k2_smem()
 {
     size_t s = (size_t)M * 4 + (size_t)S * M * 4;  // keys + state tile
-    if (RES == PF_RESAMPLE_SYSTEMATIC) s += 0;       // the scan stays in registers, the runs reuse the keys
+    if (RES == PF_RESAMPLE_SYSTEMATIC) s += (size_t)M * 4;  // the marks of the output runs
     else if (RES == PF_RESAMPLE_REFERENCE) s += (size_t)M * 4;
     else s += (size_t)M * 16;  // prob, alias, work list, scratch
     return s;
@@ -1150,6 +1133,11 @@ __device__ __forceinline__ int resample_from(const FilterDesc& D, int b, const f
     float* kb = reinterpret_cast<float*>(smem);
     float* tile = kb + M;
     unsigned char* scratch = reinterpret_cast<unsigned char*>(tile + (size_t)S * M);
+    if constexpr (RES == PF_RESAMPLE_SYSTEMATIC) {
+        // systematic_select's marks, zeroed before the barriers below
+#pragma unroll
+        for (int e = 0; e < E; ++e) reinterpret_cast<int*>(scratch)[E * tid + e] = 0;
+    }
     const bool xch = E * tid + E - 1 >= M - nx;  // this thread owns slots in the exchange range
     if constexpr (S <= 3) {
         // Small states: the sub-filter's sorted keys and state rows by bulk
@@ -1296,8 +1284,7 @@ __device__ __forceinline__ int resample_from(const FilterDesc& D, int b, const f
     if constexpr (RES == PF_RESAMPLE_SYSTEMATIC) {
         double cum[E], prev;
         const double tot = scan_f64<M, E>(w, cum, dred, &prev);
-        // the keys were read into w before the scan's barriers: kb holds the output runs
-        systematic_select<M, E>(cum, prev, ur[0] - 1.0f, tot / (double)M, reinterpret_cast<int*>(kb), sel);
+        systematic_select<M, E>(cum, prev, ur[0] - 1.0f, tot / (double)M, reinterpret_cast<int*>(scratch), sel);
     } else if constexpr (RES == PF_RESAMPLE_REFERENCE) {
         float* ex = reinterpret_cast<float*>(scratch);
 #pragma unroll
@@ -1385,8 +1372,8 @@ __global__ void __launch_bounds__(M / E, pf_min_blocks(M / E, pf_k2_warps(S))) k
 template <int M, int E, bool RANK>
 __global__ void __launch_bounds__(M / E) k_test_sort(float* keys, int32_t* idx, int32_t* fallbacks)
 {
-    __shared__ float sk[M];
-    __shared__ int si[M];
+    __shared__ __align__(16) float sk[sort_key_words(M)];
+    __shared__ __align__(16) int si[M];
     const int64_t base = (int64_t)blockIdx.x * M + E * threadIdx.x;
     float k[E];
     int ix[E];
@@ -1398,14 +1385,16 @@ __global__ void __launch_bounds__(M / E) k_test_sort(float* keys, int32_t* idx, 
     if constexpr (RANK) {
         const bool fell_back = rank_sort_desc<M, E>(k, ix, sk, si);
         if (fell_back && threadIdx.x == 0 && fallbacks) atomicAdd(fallbacks, 1);
+        // ix holds the elements' sorted positions
+#pragma unroll
+        for (int e = 0; e < E; ++e) idx[(int64_t)blockIdx.x * M + ix[e]] = E * (int)threadIdx.x + e;
     } else {
         bitonic_sort_desc<M, E>(k, ix, sk, si);
+#pragma unroll
+        for (int e = 0; e < E; ++e) idx[base + e] = ix[e];
     }
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        keys[base + e] = k[e];
-        idx[base + e] = ix[e];
-    }
+    for (int e = 0; e < E; ++e) keys[base + e] = k[e];
 }
 
 template <int M, int E, int RES>
@@ -1423,6 +1412,8 @@ __global__ void __launch_bounds__(M / E) k_test_resample(const float* w_in, cons
     int sel[E];
     if constexpr (RES == PF_RESAMPLE_SYSTEMATIC) {
         double cum[E], prev;
+#pragma unroll
+        for (int e = 0; e < E; ++e) reinterpret_cast<int*>(smem)[E * tid + e] = 0;
         const double tot = scan_f64<M, E>(w, cum, dred, &prev);
         systematic_select<M, E>(cum, prev, u[b], tot / (double)M, reinterpret_cast<int*>(smem), sel);
     } else if constexpr (RES == PF_RESAMPLE_REFERENCE) {

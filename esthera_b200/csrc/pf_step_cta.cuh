@@ -89,21 +89,19 @@ __global__ void __launch_bounds__(M / E, pf_min_blocks(M / E, pf_k1_warps(Mdl::S
     __syncthreads();  // R's shared memory and its reads of ru are done: G reuses both
 
     // ---- G (the sampling kernel's layout of shared memory)
-    unsigned char* p = smem;
-    MtgpSmem* ms = reinterpret_cast<MtgpSmem*>(p);
-    p += sizeof(MtgpSmem);
-    float* nz = reinterpret_cast<float*>(p);
+    float* nz = reinterpret_cast<float*>(smem);
     float* stage = nz;
-    p += k1_stage_bytes<Mdl, M, true>();
+    unsigned char* p = smem + k1_stage_bytes<Mdl, M, true>();
     float* sk = reinterpret_cast<float*>(p);
-    int* si = reinterpret_cast<int*>(p + (size_t)M * 4);
+    int* si = reinterpret_cast<int*>(sk + sort_key_words(M));
     {
+        auto& ms = *reinterpret_cast<K1Mtgp<Mdl, M>*>(p);
         uint32_t* gst = D.mtgp + (int64_t)b * kMtgpN;
-        mtgp_load(*ms, gst, (D.stream_base + b) % kMtgpSets, D.mask, true);
+        mtgp_load_linear<NT>(ms, gst, (D.stream_base + b) % kMtgpSets, D.mask, [] {});
         const int nbm = D.nbm;
-        mtgp_generate_bm<raw_normals<Mdl, E>()>(*ms, D.draws, nbm, nz,
-                                                [&](int k, uint32_t o) { ru[k - nbm] = __uint_as_float(o); });
-        mtgp_store(*ms, gst, D.draws);
+        const int shift = mtgp_generate_linear<raw_normals<Mdl, E>(), NT>(
+            ms, D.draws, nbm, nz, [&](int k, uint32_t o) { ru[k - nbm] = __uint_as_float(o); });
+        mtgp_store_linear(ms, gst, D.draws, shift);
     }
     __syncthreads();
 
@@ -134,31 +132,18 @@ __global__ void __launch_bounds__(M / E, pf_min_blocks(M / E, pf_k1_warps(Mdl::S
 
     // ---- S
     float k[E];
-    int ix[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        k[e] = okey[e];
-        ix[e] = E * tid + e;
-    }
-    sort_subfilter<Mdl, M, E>(k, ix, sk, si);
-    stv<E>(cur_key + base, k);
-    __syncthreads();  // normals consumed, sort buffers free: stage the state
-#pragma unroll
-    for (int v = 0; v < S; ++v)
-#pragma unroll
-        for (int e = 0; e < E; ++e) stage[v * M + E * tid + e] = st[e][v];
-    if (tid == 0) {
-        D.winner[b] = k[0];
-        s_lmax = k[0];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < S; ++v) {
-        float o[E];
-#pragma unroll
-        for (int e = 0; e < E; ++e) o[e] = stage[v * M + ix[e]];
-        stv<E>(cur_tmp + v * T + base, o);
-    }
+    for (int e = 0; e < E; ++e) k[e] = okey[e];
+    sort_subfilter<Mdl, M, E, 1>(
+        k, st, sk, si, stage,
+        [&] {
+            stv<E>(cur_key + base, k);
+            if (tid == 0) {
+                D.winner[b] = k[0];
+                s_lmax = k[0];
+            }
+        },
+        [&](int v, const float(&o)[E]) { stv<E>(cur_tmp + v * T + base, o); });
     write_partials<Mdl, E, NT, k1_stage_bytes<Mdl, M, true>()>(D, b, D.log_weights ? s_lmax : 0.0f, okey, st, sn,
                                                                 cs, reinterpret_cast<double*>(stage));
 
