@@ -1,4 +1,4 @@
-"""Fit and check the exponential used for resampling weights (pf_expneg in
+"""Fit and check the exponential used for resampling weights (pf_expneg2 in
 pf_device.cuh, restated as orc_expneg in the oracle).
 
 The resampling turns max-subtracted FP32 log-weights x <= 0 into linear
@@ -53,12 +53,12 @@ def fit(nodes=2000, iters=80, degree=6):
 
 
 def committed():
-    """c1..c6 of pf_expneg, from pf_device.cuh."""
+    """c1..c6 of pf_expneg2, from pf_device.cuh."""
     src = (HERE / "pf_device.cuh").read_text()
-    body = src[src.index("float pf_expneg(float x)"):]
+    body = src[src.index("F2 pf_expneg2(F2 x)"):]
     body = body[:body.index("return")]
-    first = float(re.search(r"float p = ([-+0-9.eE]+)f;", body).group(1))
-    rest = [float(v) for v in re.findall(r"p = fmaf\(p, r, ([-+0-9.eE]+)f\);", body)]
+    first = float(re.search(r"F2 p\(([-+0-9.eE]+)f\);", body).group(1))
+    rest = [float(v) for v in re.findall(r"p = fma2\(p, r, F2\(([-+0-9.eE]+)f\)\);", body)]
     return np.array([first] + rest[:5], np.float32)  # c6 .. c1 (the last fmaf adds the constant 1)
 
 
@@ -67,7 +67,7 @@ def fma32(a, b, c):
 
 
 def expneg32(x, coef_hi_first):
-    """The compiled sequence of pf_expneg, operation by operation in FP32."""
+    """The compiled sequence of pf_expneg2, operation by operation in FP32."""
     x = np.asarray(x, np.float32)
     with np.errstate(invalid="ignore", over="ignore"):
         return _expneg32(x, coef_hi_first)
@@ -100,7 +100,7 @@ def main(argv=None):
     ref = np.exp(x.astype(np.float64))
     ulp = np.spacing(ref.astype(np.float32)).astype(np.float64)
     err = np.abs(got - ref) / ulp
-    print("pf_expneg on [-87, 0]: max error %.2f ulp (bound %.1f), mean %.3f ulp" % (err.max(), ULP_BOUND, err.mean()))
+    print("pf_expneg2 on [-87, 0]: max error %.2f ulp (bound %.1f), mean %.3f ulp" % (err.max(), ULP_BOUND, err.mean()))
     beyond = expneg32(np.float32([-88.0, -100.0, -np.inf]), cur)
     print("below -87 and -inf ->", beyond)
     ok = err.max() <= ULP_BOUND and np.all(beyond == 0) and np.isnan(expneg32(np.float32([np.nan]), cur)[0])

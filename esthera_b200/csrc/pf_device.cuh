@@ -106,11 +106,29 @@ __device__ __forceinline__ void mtgp_store(const MtgpSmem& s, uint32_t* __restri
 // ln u1 keeps the full-precision logf: near u1 = 1 the result is tiny and an
 // approximate logarithm would lose all its relative precision.
 // ---------------------------------------------------------------------------
+// The SFU approximations without the subnormal handling of rsqrtf and
+// __fdividef (three to four instructions each around the MUFU): for normal
+// arguments -- all that the callers pass -- the same bits, compared over every
+// normal float (and mn * rcp_normal(mx) against __fdividef(mn, mx) over 2^32
+// random pairs with mn <= mx <= 2^126).
+__device__ __forceinline__ float rsqrt_normal(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_normal(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 __device__ __forceinline__ void box_muller(float x, float y, float& z1, float& z2)
 {
     const float u1 = 2.0f - x, u2 = 2.0f - y;
     const float t = -2.0f * logf(u1);
-    const float r = t > 0.0f ? t * rsqrtf(t) : 0.0f;
+    const float r = t > 0.0f ? t * rsqrt_normal(t) : 0.0f;  // t is 0 or at least 2^-23
     float s, c;
     __sincosf(kTwoPi * (u2 - 0.5f), &s, &c);
     z1 = -r * c;
@@ -186,13 +204,12 @@ __device__ __forceinline__ int mtgp_generate_linear(MtgpLinear<CAP>& s, int n, i
     const int tid = threadIdx.x;
     const uint32_t sh1 = s.sh1, sh2 = s.sh2, mask = s.mask;
     const int pos = (int)s.pos;
-    const bool odd = pos & 1;
     int shift = 0;
-    auto pair = [&](uint32_t* x, uint32_t& o0, uint32_t& o1) {
+    auto pair = [&](uint32_t* x, auto odd, uint32_t& o0, uint32_t& o1) {
         const uint2 x01 = *reinterpret_cast<const uint2*>(x);
         const uint32_t x2 = x[2];
         uint32_t t0, y0, y1;
-        if (odd) {
+        if constexpr (decltype(odd)::value) {
             const uint2 ty = *reinterpret_cast<const uint2*>(x + pos - 1);
             t0 = ty.x;
             y0 = ty.y;
@@ -219,43 +236,66 @@ __device__ __forceinline__ int mtgp_generate_linear(MtgpLinear<CAP>& s, int n, i
         o0 = (r0 >> 9) ^ s.ttb[ta & 0x0f];
         o1 = (r1 >> 9) ^ s.ttb[tb & 0x0f];
     };
-    for (int base = 0; base < n; base += kMtgpLanes) {
-        if (base - shift + kMtgpLanes > CAP) {  // the same in every thread
-            constexpr int R = (kMtgpN + NT - 1) / NT;
-            uint32_t w[R];
-#pragma unroll
-            for (int r = 0; r < R; ++r) w[r] = s.x[min(tid + r * NT, kMtgpN - 1) + base - shift];
-            __syncthreads();
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (tid + r * NT < kMtgpN) s.x[tid + r * NT] = w[r];
-            shift = base;
-            __syncthreads();
+    auto normals = [&](int k, uint32_t o0, uint32_t o1) {
+        if constexpr (RAW) {
+            *reinterpret_cast<uint2*>(nz + k) = make_uint2(o0, o1);
+        } else {
+            float z1, z2;
+            box_muller(__uint_as_float(o0), __uint_as_float(o1), z1, z2);
+            *reinterpret_cast<float2*>(nz + k) = make_float2(z1, z2);
         }
+    };
+    auto make_room = [&](int base) {
+        if (base - shift + kMtgpLanes <= CAP) return;  // the same in every thread
+        constexpr int R = (kMtgpN + NT - 1) / NT;
+        uint32_t w[R];
 #pragma unroll
-        for (int q = 0; q < PR; ++q) {
-            const int l = 2 * (tid + q * NT), k = base + l;
-            // past the requested words (the last round): nothing this pair
-            // writes is read again -- the state kept is x_n .. x_{n+350}, the
-            // last of which pair (n-2, n-1) writes
-            if (l >= kMtgpLanes || k >= n) continue;
-            uint32_t o0, o1;
-            pair(s.x + (k - shift), o0, o1);
-            if (k < nbm) {
-                if constexpr (RAW) {
-                    *reinterpret_cast<uint2*>(nz + k) = make_uint2(o0, o1);
-                } else {
-                    float z1, z2;
-                    box_muller(__uint_as_float(o0), __uint_as_float(o1), z1, z2);
-                    *reinterpret_cast<float2*>(nz + k) = make_float2(z1, z2);
-                }
-            } else {
-                emit(k, o0);
-                if (k + 1 < n) emit(k + 1, o1);
-            }
-        }
+        for (int r = 0; r < R; ++r) w[r] = s.x[min(tid + r * NT, kMtgpN - 1) + base - shift];
         __syncthreads();
-    }
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (tid + r * NT < kMtgpN) s.x[tid + r * NT] = w[r];
+        shift = base;
+        __syncthreads();
+    };
+    auto rounds = [&](auto odd) {
+        int base = 0;
+        // the rounds of normals alone: no check per word
+        for (; base + kMtgpLanes <= nbm; base += kMtgpLanes) {
+            make_room(base);
+#pragma unroll
+            for (int q = 0; q < PR; ++q) {
+                const int l = 2 * (tid + q * NT);
+                if (NT * 2 * (q + 1) > kMtgpLanes && l >= kMtgpLanes) continue;
+                uint32_t o0, o1;
+                pair(s.x + (base - shift + l), odd, o0, o1);
+                normals(base + l, o0, o1);
+            }
+            __syncthreads();
+        }
+        for (; base < n; base += kMtgpLanes) {
+            make_room(base);
+#pragma unroll 1
+            for (int q = 0; q < PR; ++q) {
+                const int l = 2 * (tid + q * NT), k = base + l;
+                // past the requested words (the last round): nothing this pair
+                // writes is read again -- the state kept is x_n .. x_{n+350},
+                // the last of which pair (n-2, n-1) writes
+                if (l >= kMtgpLanes || k >= n) continue;
+                uint32_t o0, o1;
+                pair(s.x + (k - shift), odd, o0, o1);
+                if (k < nbm) {
+                    normals(k, o0, o1);
+                } else {
+                    emit(k, o0);
+                    if (k + 1 < n) emit(k + 1, o1);
+                }
+            }
+            __syncthreads();
+        }
+    };
+    if (pos & 1) rounds(std::true_type{});
+    else rounds(std::false_type{});
     return shift;
 }
 
@@ -273,11 +313,16 @@ __device__ __forceinline__ void mtgp_store_linear(const MtgpLinear<CAP>& s, uint
 // (max error 1.4e-7 in FP32 Horner) -- plus octant reduction with one fast
 // division.  Max absolute error about 3e-7 rad.  fit_atan2.py (beside this
 // file) regenerates the fit and checks both bounds against FP64 atan2.
+// mn / mx for 0 <= mn <= mx < 2^126, 0 for mx = 0; atan2's ratio.  (A
+// subnormal mx -- both coordinates below 1.2e-38 -- is taken as 2^-126.)
+__device__ __forceinline__ float pf_ratio(float mn, float mx)
+{
+    return mn * rcp_normal(fmaxf(mx, 1.17549435e-38f));
+}
 __device__ __forceinline__ float pf_atan2(float y, float x)
 {
     const float ax = fabsf(x), ay = fabsf(y);
-    const float mx = fmaxf(ax, ay), mn = fminf(ax, ay);
-    const float a = mx > 0.0f ? __fdividef(mn, mx) : 0.0f;
+    const float a = pf_ratio(fminf(ax, ay), fmaxf(ax, ay));
     const float s = a * a;
     float p = -4.054567008e-03f;
     p = fmaf(p, s, 2.186295757e-02f);
@@ -293,6 +338,44 @@ __device__ __forceinline__ float pf_atan2(float y, float x)
     return copysignf(r, y);
 }
 
+// Two particles' FP32 values in one 64-bit register pair: the packed multiply
+// and add instructions round each half as the scalar ones do (the same bits)
+// in one issue slot.  The sampling kernels are bound by issue slots.
+struct F2 {
+    unsigned long long v;
+    __device__ __forceinline__ F2() {}
+    __device__ __forceinline__ F2(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
+    __device__ __forceinline__ explicit F2(float a) : F2(a, a) {}
+    __device__ __forceinline__ explicit F2(float2 a) : F2(a.x, a.y) {}
+    __device__ __forceinline__ void get(float& a, float& b) const
+    {
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    }
+};
+// Neither operand may be a product: the assembler fuses a packed multiply with
+// the packed add that takes its result (and with fma2(product, 1, b)) whatever
+// -fmad says.  Subtract instead: fma2(b, -1, product) keeps both roundings.
+__device__ __forceinline__ F2 operator+(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+// a - b (one rounding, as the scalar subtraction)
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, F2(-1.0f), a); }
+
 // exp(x) for the resampling's max-subtracted log-weights x <= 0, from
 // correctly rounded FP32 operations only (no SFU approximation), so that the
 // oracle's restatement (orc_expneg) gives the same bits and resampling is
@@ -301,26 +384,84 @@ __device__ __forceinline__ float pf_atan2(float y, float x)
 // this project (least squares + Lawson iterations on [-ln2/2, ln2/2],
 // relative error 2.3e-9; fit_exp.py beside this file regenerates and checks
 // it: at most 2 ulp on [-87, 0]).  x < -87 (and -inf) gives 0, NaN stays NaN.
-__device__ __forceinline__ float pf_expneg(float x)
+// Two values to a packed instruction; adding 1.5 2^23 rounds x log2 e to the
+// integer n (|n| <= 126 here) and leaves n in the sum's low bits.
+__device__ __forceinline__ F2 pf_expneg2(F2 x)
 {
-    const float n = rintf(x * 1.442695022e+00f);
-    float r = fmaf(n, -0.693145751953125f, x);
-    r = fmaf(n, -1.428606765e-06f, r);
-    float p = 1.384175848e-03f;
-    p = fmaf(p, r, 8.375782520e-03f);
-    p = fmaf(p, r, 4.166811332e-02f);
-    p = fmaf(p, r, 1.666641235e-01f);
-    p = fmaf(p, r, 4.999999404e-01f);
-    p = fmaf(p, r, 1.000000000e+00f);
-    p = fmaf(p, r, 1.0f);
-    const int ni = (int)n;
-    const bool ok = x >= -87.0f && ni >= -126;
-    const float scale = __int_as_float((ok ? ni + 127 : 0) << 23);
-    return x != x ? x : (ok ? p * scale : 0.0f);
+    const F2 t = sub2(x * F2(1.442695022e+00f), F2(-12582912.0f));
+    const F2 n = t + F2(-12582912.0f);
+    F2 r = fma2(n, F2(-0.693145751953125f), x);
+    r = fma2(n, F2(-1.428606765e-06f), r);
+    F2 p(1.384175848e-03f);
+    p = fma2(p, r, F2(8.375782520e-03f));
+    p = fma2(p, r, F2(4.166811332e-02f));
+    p = fma2(p, r, F2(1.666641235e-01f));
+    p = fma2(p, r, F2(4.999999404e-01f));
+    p = fma2(p, r, F2(1.000000000e+00f));
+    p = fma2(p, r, F2(1.0f));
+    float t0, t1, x0, x1, y0, y1;
+    t.get(t0, t1);
+    x.get(x0, x1);
+    (p * F2(__int_as_float((__float_as_int(t0) << 23) + (127 << 23)),
+            __int_as_float((__float_as_int(t1) << 23) + (127 << 23))))
+        .get(y0, y1);
+    return F2(x0 < -87.0f ? 0.0f : y0, x1 < -87.0f ? 0.0f : y1);
+}
+template <int E>
+__device__ __forceinline__ void pf_expneg_row(float (&w)[E], float mx)  // w = exp(w - mx)
+{
+    if constexpr (E == 1) {
+        float unused;
+        pf_expneg2(F2(w[0] - mx, 0.0f)).get(w[0], unused);
+    } else {
+#pragma unroll
+        for (int e = 0; e < E; e += 2) pf_expneg2(F2(w[e], w[e + 1]) + F2(-mx)).get(w[e], w[e + 1]);
+    }
+}
+
+// pf_sqrt and pf_atan2 of both halves, and the sines and cosines.
+__device__ __forceinline__ F2 pf_sqrt2(F2 d2)
+{
+    float a, b;
+    d2.get(a, b);
+    return d2 * F2(rsqrt_normal(fmaxf(a, 1e-30f)), rsqrt_normal(fmaxf(b, 1e-30f)));
+}
+__device__ __forceinline__ F2 pf_atan2_2(F2 y, F2 x)
+{
+    float y0, y1, x0, x1;
+    y.get(y0, y1);
+    x.get(x0, x1);
+    const float ax0 = fabsf(x0), ay0 = fabsf(y0), ax1 = fabsf(x1), ay1 = fabsf(y1);
+    const F2 a(pf_ratio(fminf(ax0, ay0), fmaxf(ax0, ay0)), pf_ratio(fminf(ax1, ay1), fmaxf(ax1, ay1)));
+    const F2 s = a * a;
+    F2 p(-4.054567008e-03f);
+    p = fma2(p, s, F2(2.186295757e-02f));
+    p = fma2(p, s, F2(-5.591232720e-02f));
+    p = fma2(p, s, F2(9.642197449e-02f));
+    p = fma2(p, s, F2(-1.390862965e-01f));
+    p = fma2(p, s, F2(1.994656569e-01f));
+    p = fma2(p, s, F2(-3.332986079e-01f));
+    p = fma2(p, s, F2(9.999993356e-01f));
+    float r0, r1;
+    (a * p).get(r0, r1);
+    if (ay0 > ax0) r0 = 1.57079632679489662f - r0;
+    if (ay1 > ax1) r1 = 1.57079632679489662f - r1;
+    if (x0 < 0.0f) r0 = kPi - r0;
+    if (x1 < 0.0f) r1 = kPi - r1;
+    return F2(copysignf(r0, y0), copysignf(r1, y1));
+}
+__device__ __forceinline__ void sincos2(F2 a, F2& sn, F2& cs)
+{
+    float a0, a1, s0, s1, c0, c1;
+    a.get(a0, a1);
+    __sincosf(a0, &s0, &c0);
+    __sincosf(a1, &s1, &c1);
+    sn = F2(s0, s1);
+    cs = F2(c0, c1);
 }
 
 // sqrt(d2) for d2 >= 0 through the SFU reciprocal square root (0 -> 0).
-__device__ __forceinline__ float pf_sqrt(float d2) { return d2 * rsqrtf(fmaxf(d2, 1e-30f)); }
+__device__ __forceinline__ float pf_sqrt(float d2) { return d2 * rsqrt_normal(fmaxf(d2, 1e-30f)); }
 
 // E consecutive 4-byte values of shared memory at once (p aligned to 4E bytes
 // where E is 2 or a multiple of 4).
@@ -571,7 +712,10 @@ __device__ __forceinline__ bool rank_sort_desc(float (&k)[E], int (&pos)[E], flo
 #pragma unroll
         for (int step = M / 2; step > 0; step >>= 1) {
             const int up = step >= 32 ? step + step / 32 : step;
-            if (sk[q + pad(step - 1)] > k[e]) q += up;
+            // (one predicated add per level)
+            asm("{\n.reg .pred p;\nsetp.gt.f32 p, %1, %2;\n@p add.s32 %0, %0, %3;\n}"
+                : "+r"(q)
+                : "f"(sk[q + pad(step - 1)]), "f"(k[e]), "r"(up));
         }
         pos[e] = q - ((q * 993) >> 15);  // q - q / 33 (q < 33 * 993)
     }
@@ -593,6 +737,23 @@ __device__ __forceinline__ float block_max(float v, float* red)
     float r = red[0];
     for (int i = 1; i < nw; ++i) r = fmaxf(r, red[i]);
     return r;
+}
+
+// The largest of the CTA's keys (NT threads, E each; NaN keys ignored), the same
+// in every thread.  red: NT / 32 floats.  One barrier.
+template <int NT, int E>
+__device__ __forceinline__ float cta_max(const float (&k)[E], float* red)
+{
+    float v = k[0];
+#pragma unroll
+    for (int e = 1; e < E; ++e) v = fmaxf(v, k[e]);
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(v) : "f"(v));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = red[0];
+#pragma unroll
+    for (int w = 1; w < NT / 32; ++w) v = fmaxf(v, red[w]);
+    return v;
 }
 
 // Canonical FP64 inclusive scan (the oracle's orc_scan_f64): each thread sums
@@ -676,10 +837,10 @@ __device__ __forceinline__ int upper_count(const double* cum, double x)
 // pos(i)), so every output selects the same input (pos is non-decreasing in
 // i).  Synchronises the CTA.
 //
-// Bound: latency (FP64 conversions and comparisons in a chain per boundary).
-// At m = 512, 4 particles per thread a CTA of a full grid spends 2870 cycles
-// here, against 3840 when each thread wrote its inputs' runs out one by one --
-// a heavy particle's run is hundreds of outputs long -- after an FP64 division.
+// Bound: issue slots.  Measured with the rest of the resampling kernel: 6M
+// particles in sub-filters of 256, 6274 -> 5957 us per 32 steps for boundaries
+// from one FP64 estimate each (pos() evaluated only near an integer) and the
+// packed exponentials, against two evaluations of pos() per boundary.
 template <int M, int E>
 __device__ __forceinline__ void systematic_select(const double (&cum)[E], double prev, float u0f, double step,
                                                   int* mark, int (&sel)[E])
@@ -687,37 +848,58 @@ __device__ __forceinline__ void systematic_select(const double (&cum)[E], double
     const int tid = threadIdx.x;
     constexpr int W = 32 * E;  // outputs of a warp
     const double u0 = (double)u0f;
-    // 1 / step for the estimates only: a Newton step from the FP32 reciprocal
-    // (about 1e-13) where that neither over- nor underflows
-    const float sf = (float)step;
-    double inv;
-    if (sf > 1e-30f && sf < 1e30f) {
-        inv = (double)__frcp_rn(sf);
-        inv = fma(inv, fma(-step, inv, 1.0), inv);
-    } else {
-        inv = step > 0.0 ? 1.0 / step : 0.0;
-    }
     auto pos = [&](int i) { return (u0 + (double)i) * step; };
-    auto first_at_or_above = [&](double t) {  // first i in [0, M] with pos(i) >= t
-        const double est = fma(t, inv, -u0);
-        int i = est > 0.0 ? (est < (double)M ? __double2int_ru(est) : M) : 0;
-        if ((i > 0 && pos(i - 1) >= t) || (i < M && pos(i) < t)) {  // the estimate is off: rarely
-            while (i > 0 && pos(i - 1) >= t) --i;
-            while (i < M && pos(i) < t) ++i;
-        }
+    auto exact = [&](int i, double t) {  // first i in [0, M] with pos(i) >= t, from any start
+        while (i > 0 && pos(i - 1) >= t) --i;
+        while (i < M && pos(i) < t) ++i;
         return i;
     };
     const int j0 = E * tid;
-    int lo = j0 == 0 ? 0 : first_at_or_above(prev);
+    int first[E + 1];  // first output at or above the sum before input j0 + e
+    // 1 / step by two Newton steps from the FP32 reciprocal of its mantissa: t /
+    // step - u0 below is then within 1e-11 of the truth, and so are the rounded
+    // pos(i)
+    const int hw = __double2hiint(step), ex = hw >> 20;
+    if (ex >= 200 && ex <= 1800) {  // any positive sum of FP32 weights
+        const double sm = __hiloint2double((hw & 0xfffff) | (1023 << 20), __double2loint(step));
+        double inv = (double)rcp_normal((float)sm);
+        inv = fma(inv, fma(-sm, inv, 1.0), inv);
+        inv = fma(inv, fma(-sm, inv, 1.0), inv) * __hiloint2double((2046 - ex) << 20, 0);
+        bool close = false;
+        auto guess = [&](double t) {
+            // x to the nearest integer (in the low word of x + 1.5 2^52), and
+            // the distance to it: unless that is below 2^-20 the ceiling of x
+            // is the answer, without evaluating pos
+            const double x = fma(t, inv, -u0);
+            const double r = x + 6755399441055744.0;
+            const int d = __double2hiint(x - (r - 6755399441055744.0));
+            close |= (d & 0x7fffffff) < (1003 << 20);
+            return min(max(__double2loint(r) + (d >= 0 ? 1 : 0), 0), M);
+        };
+        first[0] = j0 == 0 ? 0 : guess(prev);
+#pragma unroll
+        for (int e = 0; e < E; ++e) first[e + 1] = guess(cum[e]);
+        if (close) {
+            if (j0 != 0) first[0] = exact(first[0], prev);
+#pragma unroll
+            for (int e = 0; e < E; ++e) first[e + 1] = exact(first[e + 1], cum[e]);
+        }
+    } else {  // all weights zero, or a sum that is not finite
+        first[0] = j0 == 0 ? 0 : exact(0, prev);
+#pragma unroll 1
+        for (int e = 0; e < E; ++e) first[e + 1] = exact(0, cum[e]);
+    }
+    if (j0 + E == M) first[E] = M;
+    int lo = first[0];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-        const int j = j0 + e;
-        const int hi = j == M - 1 ? M : first_at_or_above(cum[e]);
+        const int hi = first[e + 1];
         if (lo < hi) {
-            mark[lo] = j;
-            for (int i = (lo / W + 1) * W; i < hi; i += W) mark[i] = j;
+            mark[lo] = j0 + e;
+            if ((lo ^ (hi - 1)) >= W)
+                for (int i = (lo / W + 1) * W; i < hi; i += W) mark[i] = j0 + e;
         }
-        lo = hi > lo ? hi : lo;
+        lo = max(lo, hi);
     }
     __syncthreads();
 #pragma unroll
@@ -1065,6 +1247,12 @@ union ModelParams {
 };
 
 __device__ __forceinline__ float wrap_pi(float a) { return fmaf(-kTwoPi, floorf((a + kPi) * kInvTwoPi), a); }
+__device__ __forceinline__ F2 wrap_pi2(F2 a)
+{
+    float k0, k1;
+    ((a + F2(kPi)) * F2(kInvTwoPi)).get(k0, k1);
+    return fma2(F2(-kTwoPi), F2(floorf(k0), floorf(k1)), a);
+}
 
 struct Unicycle {
     static constexpr int S = 3, K = 3, NA = 1, C = 2, Z = 16;
@@ -1072,7 +1260,10 @@ struct Unicycle {
     struct Consts {
         float A, B, wd, sq0, sq1, sq2, isr, isb;
         int L;
-        float lx[8], ly[8], rm[8], cb[8], sb[8];
+        // each value twice (a packed operand), two to a 16-byte load
+        struct alignas(16) Landmark {
+            float2 lx, ly, cb, sb, nsb, rm;
+        } lm[8];
     };
     // Exact-arc velocity model: x' = x + A cos th - B sin th, y' = y + A sin th + B cos th
     // with A = v sin(w dt)/w, B = v (1 - cos(w dt))/w (straight-line limit as w -> 0),
@@ -1108,10 +1299,15 @@ struct Unicycle {
             c.L = L;
         } else if (lane < 8) {
             const int j = lane;
-            c.lx[j] = p.landmarks[j][0];
-            c.ly[j] = p.landmarks[j][1];
-            c.rm[j] = j < L ? in.meas[j] : 0.0f;
-            sincosf(j < L ? in.meas[L + j] : 0.0f, &c.sb[j], &c.cb[j]);
+            const float x = p.landmarks[j][0], y = p.landmarks[j][1], r = j < L ? in.meas[j] : 0.0f;
+            float sb, cb;
+            sincosf(j < L ? in.meas[L + j] : 0.0f, &sb, &cb);
+            c.lm[j].lx = make_float2(x, x);
+            c.lm[j].ly = make_float2(y, y);
+            c.lm[j].rm = make_float2(r, r);
+            c.lm[j].cb = make_float2(cb, cb);
+            c.lm[j].sb = make_float2(sb, sb);
+            c.lm[j].nsb = make_float2(-sb, -sb);
         }
     }
     __device__ static __forceinline__ float step(const Consts& c, float* s, const float* n, float* sn,
@@ -1133,11 +1329,11 @@ struct Unicycle {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             if (j < c.L) {
-                const float dx = c.lx[j] - nx, dy = c.ly[j] - ny;
+                const float dx = c.lm[j].lx.x - nx, dy = c.lm[j].ly.x - ny;
                 const float r = pf_sqrt(fmaf(dx, dx, dy * dy));
-                const float er = (c.rm[j] - r) * c.isr;
-                const float cp = fmaf(c2, c.cb[j], -(s2 * c.sb[j]));
-                const float sp = fmaf(s2, c.cb[j], c2 * c.sb[j]);
+                const float er = (c.lm[j].rm.x - r) * c.isr;
+                const float cp = fmaf(c2, c.lm[j].cb.x, -(s2 * c.lm[j].sb.x));
+                const float sp = fmaf(s2, c.lm[j].cb.x, c2 * c.lm[j].sb.x);
                 const float eb = pf_atan2(fmaf(sp, dx, -(cp * dy)), fmaf(cp, dx, sp * dy)) * c.isb;
                 acc = fmaf(er, er, acc);
                 acc = fmaf(eb, eb, acc);
@@ -1166,11 +1362,11 @@ struct Unicycle {
         float acc = 0.0f;
 #pragma unroll 1
         for (int j = h; j < c.L; j += 2) {
-            const float dx = c.lx[j] - nx, dy = c.ly[j] - ny;
+            const float dx = c.lm[j].lx.x - nx, dy = c.lm[j].ly.x - ny;
             const float r = pf_sqrt(fmaf(dx, dx, dy * dy));
-            const float er = (c.rm[j] - r) * c.isr;
-            const float cp = fmaf(c2, c.cb[j], -(s2 * c.sb[j]));
-            const float sp = fmaf(s2, c.cb[j], c2 * c.sb[j]);
+            const float er = (c.lm[j].rm.x - r) * c.isr;
+            const float cp = fmaf(c2, c.lm[j].cb.x, -(s2 * c.lm[j].sb.x));
+            const float sp = fmaf(s2, c.lm[j].cb.x, c2 * c.lm[j].sb.x);
             const float eb = pf_atan2(fmaf(sp, dx, -(cp * dy)), fmaf(cp, dx, sp * dy)) * c.isb;
             acc = fmaf(er, er, acc);
             acc = fmaf(eb, eb, acc);
@@ -1179,49 +1375,64 @@ struct Unicycle {
         return -0.5f * (h ? o + acc : acc + o);
     }
     // E particles at once: the same per-particle arithmetic as step() in the
-    // same order (bit-identical results), with the landmark loop outside the
+    // same order (bit-identical results), two particles to a packed
+    // instruction (F2) where E is even, with the landmark loop outside the
     // particle loop so each landmark's constants are read once per thread and
-    // the E likelihood chains interleave.  noise(e, v) gives particle e's v-th
+    // the likelihood chains interleave.  noise(e, v) gives particle e's v-th
     // normal.
     template <int E, class Noise>
     __device__ static __forceinline__ void step_batch(const Consts& c, float (&s)[E][S], Noise noise,
                                                       float (&sn)[E][NA], float (&cs)[E][NA], float (&ll)[E])
     {
-        float s2[E], c2[E], acc[E];
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            float st, ct;
-            __sincosf(s[e][2], &st, &ct);
-            const float nx = fmaf(c.sq0, noise(e, 0), fmaf(c.A, ct, fmaf(-c.B, st, s[e][0])));
-            const float ny = fmaf(c.sq1, noise(e, 1), fmaf(c.A, st, fmaf(c.B, ct, s[e][1])));
-            const float nt = wrap_pi(fmaf(c.sq2, noise(e, 2), s[e][2] + c.wd));
-            s[e][0] = nx;
-            s[e][1] = ny;
-            s[e][2] = nt;
-            __sincosf(nt, &s2[e], &c2[e]);
-            sn[e][0] = s2[e];
-            cs[e][0] = c2[e];
-            acc[e] = 0.0f;
-        }
-        const int L = c.L;
-        const float isr = c.isr, isb = c.isb;
-#pragma unroll 1
-        for (int j = 0; j < L; ++j) {
-            const float lx = c.lx[j], ly = c.ly[j], rm = c.rm[j], cb = c.cb[j], sb = c.sb[j];
+        if constexpr (E % 2 != 0) {
 #pragma unroll
             for (int e = 0; e < E; ++e) {
-                const float dx = lx - s[e][0], dy = ly - s[e][1];
-                const float r = pf_sqrt(fmaf(dx, dx, dy * dy));
-                const float er = (rm - r) * isr;
-                const float cp = fmaf(c2[e], cb, -(s2[e] * sb));
-                const float sp = fmaf(s2[e], cb, c2[e] * sb);
-                const float eb = pf_atan2(fmaf(sp, dx, -(cp * dy)), fmaf(cp, dx, sp * dy)) * isb;
-                acc[e] = fmaf(er, er, acc[e]);
-                acc[e] = fmaf(eb, eb, acc[e]);
+                const float n[K] = {noise(e, 0), noise(e, 1), noise(e, 2)};
+                ll[e] = step(c, s[e], n, sn[e], cs[e]);
             }
-        }
+        } else {
+            constexpr int P = E / 2;
+            F2 x[P], y[P], s2[P], c2[P], acc[P];
 #pragma unroll
-        for (int e = 0; e < E; ++e) ll[e] = -0.5f * acc[e];
+            for (int q = 0; q < P; ++q) {
+                const int e = 2 * q;
+                const F2 th(s[e][2], s[e + 1][2]);
+                F2 st, ct;
+                sincos2(th, st, ct);
+                x[q] = fma2(F2(c.sq0), F2(noise(e, 0), noise(e + 1, 0)),
+                            fma2(F2(c.A), ct, fma2(F2(-c.B), st, F2(s[e][0], s[e + 1][0]))));
+                y[q] = fma2(F2(c.sq1), F2(noise(e, 1), noise(e + 1, 1)),
+                            fma2(F2(c.A), st, fma2(F2(c.B), ct, F2(s[e][1], s[e + 1][1]))));
+                const F2 nt = wrap_pi2(fma2(F2(c.sq2), F2(noise(e, 2), noise(e + 1, 2)), th + F2(c.wd)));
+                x[q].get(s[e][0], s[e + 1][0]);
+                y[q].get(s[e][1], s[e + 1][1]);
+                nt.get(s[e][2], s[e + 1][2]);
+                sincos2(nt, s2[q], c2[q]);
+                s2[q].get(sn[e][0], sn[e + 1][0]);
+                c2[q].get(cs[e][0], cs[e + 1][0]);
+                acc[q] = F2(0.0f);
+            }
+            const int L = c.L;
+            const F2 isr(c.isr), isb(c.isb);
+#pragma unroll 1
+            for (int j = 0; j < L; ++j) {
+                const typename Consts::Landmark m = c.lm[j];
+                const F2 lx(m.lx), ly(m.ly), rm(m.rm), cb(m.cb), sb(m.sb), nsb(m.nsb);
+#pragma unroll
+                for (int q = 0; q < P; ++q) {
+                    const F2 dx = sub2(lx, x[q]), dy = sub2(ly, y[q]), ndy = dy * F2(-1.0f);
+                    const F2 r = pf_sqrt2(fma2(dx, dx, dy * dy));
+                    const F2 er = sub2(rm, r) * isr;
+                    const F2 cp = fma2(c2[q], cb, s2[q] * nsb);
+                    const F2 sp = fma2(s2[q], cb, c2[q] * sb);
+                    const F2 eb = pf_atan2_2(fma2(sp, dx, cp * ndy), fma2(cp, dx, sp * dy)) * isb;
+                    acc[q] = fma2(er, er, acc[q]);
+                    acc[q] = fma2(eb, eb, acc[q]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < P; ++q) (F2(-0.5f) * acc[q]).get(ll[2 * q], ll[2 * q + 1]);
+        }
     }
 };
 
@@ -1229,8 +1440,12 @@ struct DhArm {
     static constexpr int S = 12, K = 6, NA = 6, C = 0, Z = 6;
     __host__ __device__ static constexpr int angle_var(int a) { return a; }
     struct Consts {
+        // each value twice (a packed operand), two to a 16-byte load
+        struct alignas(16) Joint {
+            float2 a, d, ca, sa, nca, nsa;
+        } j[6];
         float dt, sqd, isp, isa;
-        float a[6], d[6], ca[6], sa[6], z[6];
+        float z[6];
     };
     // lane 6: scalars; lanes 0..5: joint `lane`
     __device__ static void prepare(Consts& c, const pf_step_input& in, const ModelParams& mp, int lane)
@@ -1243,9 +1458,10 @@ struct DhArm {
             c.isa = 1.0f / p.sigma_ang;
         } else if (lane < 6) {
             const int i = lane;
-            c.a[i] = p.a[i];
-            c.d[i] = p.d[i];
-            sincosf(p.alpha[i], &c.sa[i], &c.ca[i]);
+            float sa, ca;
+            sincosf(p.alpha[i], &sa, &ca);
+            c.j[i] = {make_float2(p.a[i], p.a[i]), make_float2(p.d[i], p.d[i]), make_float2(ca, ca),
+                      make_float2(sa, sa), make_float2(-ca, -ca), make_float2(-sa, -sa)};
             c.z[i] = in.meas[i];
         }
     }
@@ -1264,10 +1480,10 @@ struct DhArm {
             sn[i] = sq;
             cs[i] = cq;
             // A_i = [[c, -s ca, s sa, a c], [s, c ca, -c sa, a s], [0, sa, ca, d]]
-            const float a00 = cq, a01 = -(sq * c.ca[i]), a02 = sq * c.sa[i];
-            const float a10 = sq, a11 = cq * c.ca[i], a12 = -(cq * c.sa[i]);
-            const float a21 = c.sa[i], a22 = c.ca[i];
-            const float t0 = c.a[i] * cq, t1 = c.a[i] * sq, t2 = c.d[i];
+            const float a00 = cq, a01 = -(sq * c.j[i].ca.x), a02 = sq * c.j[i].sa.x;
+            const float a10 = sq, a11 = cq * c.j[i].ca.x, a12 = -(cq * c.j[i].sa.x);
+            const float a21 = c.j[i].sa.x, a22 = c.j[i].ca.x;
+            const float t0 = c.j[i].a.x * cq, t1 = c.j[i].a.x * sq, t2 = c.j[i].d.x;
             const float n00 = fmaf(R01, a10, R00 * a00), n01 = fmaf(R02, a21, fmaf(R01, a11, R00 * a01)),
                         n02 = fmaf(R02, a22, fmaf(R01, a12, R00 * a02));
             const float n10 = fmaf(R11, a10, R10 * a00), n11 = fmaf(R12, a21, fmaf(R11, a11, R10 * a01)),
@@ -1297,6 +1513,72 @@ struct DhArm {
         acc = fmaf(d5, d5, acc);
         return -0.5f * acc;
     }
+    // E particles at once (E even): step()'s arithmetic in the same order for
+    // two particles to a packed instruction (F2), bit-identical results.
+    template <int E, class Noise>
+    __device__ static __forceinline__ void step_batch(const Consts& c, float (&s)[E][S], Noise noise,
+                                                      float (&sn)[E][NA], float (&cs)[E][NA], float (&ll)[E])
+    {
+        if constexpr (E % 2 != 0) {
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                float n[K];
+#pragma unroll
+                for (int v = 0; v < K; ++v) n[v] = noise(e, v);
+                ll[e] = step(c, s[e], n, sn[e], cs[e]);
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < E; e += 2) {
+                F2 R[9], p[3];
+#pragma unroll
+                for (int i = 0; i < 9; ++i) R[i] = F2(i % 4 == 0 ? 1.0f : 0.0f);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) p[i] = F2(0.0f);
+#pragma unroll
+                for (int i = 0; i < 6; ++i) {
+                    const F2 v(s[e][6 + i], s[e + 1][6 + i]);
+                    const F2 q = wrap_pi2(fma2(v, F2(c.dt), F2(s[e][i], s[e + 1][i])));
+                    q.get(s[e][i], s[e + 1][i]);
+                    fma2(F2(c.sqd), F2(noise(e, i), noise(e + 1, i)), v).get(s[e][6 + i], s[e + 1][6 + i]);
+                    F2 sq, cq;
+                    sincos2(q, sq, cq);
+                    sq.get(sn[e][i], sn[e + 1][i]);
+                    cq.get(cs[e][i], cs[e + 1][i]);
+                    const typename Consts::Joint j = c.j[i];
+                    const F2 a01 = sq * F2(j.nca), a02 = sq * F2(j.sa);
+                    const F2 a11 = cq * F2(j.ca), a12 = cq * F2(j.nsa);
+                    const F2 t0 = F2(j.a) * cq, t1 = F2(j.a) * sq;
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) {
+                        const F2 r0 = R[3 * r], r1 = R[3 * r + 1], r2 = R[3 * r + 2];
+                        p[r] = fma2(r2, F2(j.d), fma2(r1, t1, fma2(r0, t0, p[r])));
+                        R[3 * r] = fma2(r1, sq, r0 * cq);
+                        R[3 * r + 1] = fma2(r2, F2(j.sa), fma2(r1, a11, r0 * a01));
+                        R[3 * r + 2] = fma2(r2, F2(j.ca), fma2(r1, a12, r0 * a02));
+                    }
+                }
+                const F2 yaw = pf_atan2_2(R[3], R[0]);
+                const F2 pitch = pf_atan2_2(R[6] * F2(-1.0f), pf_sqrt2(fma2(R[7], R[7], R[8] * R[8])));
+                const F2 roll = pf_atan2_2(R[7], R[8]);
+                F2 acc(0.0f);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const F2 d = sub2(F2(c.z[i]), p[i]) * F2(c.isp);
+                    acc = i == 0 ? d * d : fma2(d, d, acc);
+                }
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    F2 d = sub2(F2(c.z[3 + i]), i == 0 ? yaw : (i == 1 ? pitch : roll));
+                    float k0, k1;
+                    (d * F2(kInvTwoPi)).get(k0, k1);
+                    d = fma2(F2(-kTwoPi), F2(rintf(k0), rintf(k1)), d) * F2(c.isa);
+                    acc = fma2(d, d, acc);
+                }
+                (F2(-0.5f) * acc).get(ll[e], ll[e + 1]);
+            }
+        }
+    }
     // Two threads per particle (lane pair h = 0, 1): both lanes advance all
     // joints (identical arithmetic); lane h chains the transforms of joints
     // 3h .. 3h+2 from the identity, the pair swaps chains and joint sines, and
@@ -1323,11 +1605,11 @@ struct DhArm {
             __sincosf(qi, &sq, &cq);
             msn[k] = sq;
             mcs[k] = cq;
-            const float ca = c.ca[i], sa = c.sa[i];
+            const float ca = c.j[i].ca.x, sa = c.j[i].sa.x;
             const float a00 = cq, a01 = -(sq * ca), a02 = sq * sa;
             const float a10 = sq, a11 = cq * ca, a12 = -(cq * sa);
             const float a21 = sa, a22 = ca;
-            const float t0 = c.a[i] * cq, t1 = c.a[i] * sq, t2 = c.d[i];
+            const float t0 = c.j[i].a.x * cq, t1 = c.j[i].a.x * sq, t2 = c.j[i].d.x;
             float N[9];
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
@@ -1626,14 +1908,14 @@ struct Beacon {
         return fmaf(-c.h, h ? o + acc : acc + o, c.lnorm);
     }
     // E particles at once: step()'s per-particle arithmetic in the same order
-    // (bit-identical results), the beacon loop outside the particle loop so
-    // each beacon's constants are read once per thread and the E range
-    // chains interleave.  noise(e, v) gives particle e's v-th normal.
+    // (bit-identical results), two particles to a packed instruction in the
+    // beacon loop where E is even; the loop outside the particle loop so each
+    // beacon's constants are read once per thread and the range chains
+    // interleave.  noise(e, v) gives particle e's v-th normal.
     template <int E, class Noise>
     __device__ static __forceinline__ void step_batch(const Consts& c, float (&s)[E][S], Noise noise,
                                                       float (&sn)[E][NA], float (&cs)[E][NA], float (&ll)[E])
     {
-        float acc[E];
 #pragma unroll
         for (int e = 0; e < E; ++e) {
             const float v = fmaf(c.nv, noise(e, 0), c.v);
@@ -1650,21 +1932,43 @@ struct Beacon {
             s[e][1] = ny;
             s[e][2] = nt;
             __sincosf(nt, &sn[e][0], &cs[e][0]);
-            acc[e] = 0.0f;
         }
         const int L = c.L;
-#pragma unroll 1
-        for (int j = 0; j < L; ++j) {
-            const float bx = c.bx[j], by = c.by[j], bz2 = c.bz2[j], z = c.z[j];
+        if constexpr (E % 2 != 0) {
 #pragma unroll
             for (int e = 0; e < E; ++e) {
-                const float dx = s[e][0] - bx, dy = s[e][1] - by;
-                const float r = pf_sqrt(fmaf(dx, dx, fmaf(dy, dy, bz2))) - z;
-                acc[e] = fmaf(r, r, acc[e]);
+                float acc = 0.0f;
+#pragma unroll 1
+                for (int j = 0; j < L; ++j) {
+                    const float dx = s[e][0] - c.bx[j], dy = s[e][1] - c.by[j];
+                    const float r = pf_sqrt(fmaf(dx, dx, fmaf(dy, dy, c.bz2[j]))) - c.z[j];
+                    acc = fmaf(r, r, acc);
+                }
+                ll[e] = fmaf(-c.h, acc, c.lnorm);
             }
-        }
+        } else {
+            constexpr int P = E / 2;
+            F2 x[P], y[P], acc[P];
 #pragma unroll
-        for (int e = 0; e < E; ++e) ll[e] = fmaf(-c.h, acc[e], c.lnorm);
+            for (int q = 0; q < P; ++q) {
+                x[q] = F2(s[2 * q][0], s[2 * q + 1][0]);
+                y[q] = F2(s[2 * q][1], s[2 * q + 1][1]);
+                acc[q] = F2(0.0f);
+            }
+#pragma unroll 1
+            for (int j = 0; j < L; ++j) {
+                const F2 nbx(-c.bx[j]), nby(-c.by[j]), bz2(c.bz2[j]), z(c.z[j]);
+#pragma unroll
+                for (int q = 0; q < P; ++q) {
+                    const F2 dx = x[q] + nbx, dy = y[q] + nby;
+                    const F2 r = sub2(pf_sqrt2(fma2(dx, dx, fma2(dy, dy, bz2))), z);
+                    acc[q] = fma2(r, r, acc[q]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < P; ++q)
+                fma2(F2(-c.h), acc[q], F2(c.lnorm)).get(ll[2 * q], ll[2 * q + 1]);
+        }
     }
 };
 
@@ -1744,8 +2048,7 @@ struct RareTies<Beacon> : std::true_type {};
 
 // The sampling kernels' sort of one sub-filter per CTA: k[e] in, the sorted key
 // at position E*tid+e out, and the particles' state rows in sorted order into
-// stage[v * M + ..], which must be free (nothing reads it once every thread has
-// entered).  Rare ties: every particle is scattered to its sorted position
+// stage[v * M + ..] (others may still be reading it on entry).  Rare ties: every particle is scattered to its sorted position
 // (rank_sort_desc); otherwise the network's indices gather.  store(v, row) gets
 // this thread's E values of sorted row v (a pair's lanes take alternate rows);
 // sorted() runs once the keys are in order.  stage may be read by others until
@@ -1767,11 +2070,8 @@ __device__ __forceinline__ void sort_subfilter(float (&k)[E], const float (&st)[
             for (int e = 0; e < E; ++e) stage[v * M + ix[e]] = st[e][v];
         }
     } else {
-#pragma unroll
-        for (int e = 0; e < E; ++e) ix[e] = E * tid + e;
-        bitonic_sort_desc<M, E, TP>(k, ix, sk, si, tid, h == 0);
-        sorted();
-        __syncthreads();  // (a sub-filter of one warp has met no barrier since its normals were read)
+        // the rows go to shared memory first: the network needs the registers
+        __syncthreads();
         if (h == 0) {
 #pragma unroll
             for (int v = 0; v < S; ++v) {
@@ -1781,6 +2081,10 @@ __device__ __forceinline__ void sort_subfilter(float (&k)[E], const float (&st)[
                 sts_row<E>(stage + v * M + E * tid, o);
             }
         }
+#pragma unroll
+        for (int e = 0; e < E; ++e) ix[e] = E * tid + e;
+        bitonic_sort_desc<M, E, TP>(k, ix, sk, si, tid, h == 0);
+        sorted();
     }
     __syncthreads();
 #pragma unroll

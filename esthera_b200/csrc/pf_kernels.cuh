@@ -101,9 +101,10 @@ __device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcont
 // Register budgets of the split pipeline's kernels, as resident warps per SM
 // asked of the compiler: __launch_bounds__(threads, ceil(warps * 32 / threads))
 // caps the registers at 65536 / (that many threads).  Small states (the
-// unicycle's 3 variables) take 36 / 32 warps: the sampling kernel at m = 512,
-// 4 particles per thread runs 53 us capped at 56 registers against 59 us at
-// the compiler's own 83.  The arms' states (9-12 variables, forward
+// unicycle's 3 variables) take 36 / 32 warps: 16 steps of 2^20 particles (m =
+// 512, 4 particles per thread) take 517 us at 56 or 64 registers of the
+// sampling kernel, 526 us at 72; 6M particles in sub-filters of 256 take 6255
+// us at 56 and 6277 us at 64.  The arms' states (9-12 variables, forward
 // kinematics) need ~128 registers per thread; capping them lower spills.
 // The sampling kernel with two threads per particle asks for 4 warps fewer
 // (its CTAs are twice as large, so the rounding up of whole CTAs would
@@ -125,11 +126,12 @@ __host__ __device__ constexpr int pf_min_blocks(int threads, int warps)
     return (warps * 32 + threads - 1) / threads > 32 ? 32 : (warps * 32 + threads - 1) / threads;
 }
 // Large states with 2 or fewer particles per thread hold half the registers a
-// thread of 4 needs: their budget is 32 warps (64 registers; the DH arm's
-// sampling kernel at m = 256 runs 26.4 us against 29.6 us at 128 registers
-// and 28.8 us with 4 particles per thread).
+// thread of 4 needs: their budget is 28 warps (72 registers: the packed
+// kinematic chain of the DH arm at m = 256 spills less than at 64, and 2^18
+// particles still fit one wave; 16 steps of 2^18 particles 292 us, against 307
+// at 32 warps and 297 at 24).
 #ifndef PF_K1_WARPS_LARGE_E2
-#define PF_K1_WARPS_LARGE_E2 32
+#define PF_K1_WARPS_LARGE_E2 28
 #endif
 __host__ __device__ constexpr int pf_k1_warps(int S, int E = 4)
 {
@@ -272,7 +274,8 @@ constexpr size_t k1_smem()
 // at most 32) each add NT / P rows in order, then an xor-shuffle tree over
 // the P lanes.  A fixed order: deterministic for a given (M, E).  A thread
 // with counts = false (the second lane of a particle pair) adds zeros.
-template <class Mdl, int E, int NT, size_t ACC_BYTES>
+// FREE: the caller's last barrier already freed the buffer.
+template <class Mdl, int E, int NT, size_t ACC_BYTES, bool FREE = false>
 __device__ __forceinline__ void write_partials(const FilterDesc& D, int b, float lmax, const float (&okey)[E],
                                                const float (&st)[E][Mdl::S],
                                                const float (&sn)[E][Mdl::NA > 0 ? Mdl::NA : 1],
@@ -291,7 +294,7 @@ __device__ __forceinline__ void write_partials(const FilterDesc& D, int b, float
     double* out = D.part + (int64_t)b * kPartStride;
 #pragma unroll
     for (int c0 = 0; c0 < NV; c0 += CH) {
-        __syncthreads();  // the buffer (or the previous chunk) is free
+        if (!FREE || c0 > 0) __syncthreads();  // the buffer (or the previous chunk) is free
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
             const int i = c0 + c;
@@ -350,7 +353,7 @@ __global__ void __launch_bounds__(TP * M / E, pf_min_blocks(TP * M / E, pf_k1_wa
     constexpr int NANG = NA > 0 ? NA : 1;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ typename Mdl::Consts cst;
-    __shared__ float s_lmax;
+    __shared__ float s_max[NT / 32];
     __shared__ FilterDesc sdesc;
     int f, b;
     cta_target(cta_map, f, b);
@@ -418,6 +421,12 @@ __global__ void __launch_bounds__(TP * M / E, pf_min_blocks(TP * M / E, pf_k1_wa
             stv<E>(D.state + v * T + base, o);
         }
     }
+    // the partials before the sort, which then carries the keys (and the
+    // scattered rows) alone through its registers; the barrier in cta_max also
+    // frees the normals' buffer
+    const float lmax = cta_max<NT, E>(okey, s_max);
+    write_partials<Mdl, E, NT, k1_stage_bytes<Mdl, M, FR, TP>(), true>(
+        D, b, D.log_weights ? lmax : 0.0f, okey, st, sn, cs, reinterpret_cast<double*>(stage), writer);
     float k[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) k[e] = okey[e];
@@ -425,14 +434,9 @@ __global__ void __launch_bounds__(TP * M / E, pf_min_blocks(TP * M / E, pf_k1_wa
         k, st, sk, si, stage,
         [&] {
             if (writer) stv<E>(D.tkey + base, k);
-            if (tid == 0) {
-                D.winner[b] = k[0];
-                s_lmax = k[0];
-            }
+            if (tid == 0) D.winner[b] = k[0];
         },
         [&](int v, const float(&o)[E]) { stv<E>(D.tmp + v * T + base, o); });
-    write_partials<Mdl, E, NT, k1_stage_bytes<Mdl, M, FR, TP>()>(D, b, D.log_weights ? s_lmax : 0.0f, okey, st, sn,
-                                                                  cs, reinterpret_cast<double*>(stage), writer);
 }
 
 // ---------------------------------------------------------------------------
@@ -1239,17 +1243,17 @@ __device__ __forceinline__ int resample_from(const FilterDesc& D, int b, const f
         // the CTA-wide maximum); a NaN key breaks the order: then the CTA-wide one
         const int nxc = exchange_count(D);
         float mx;
-        if (!any_nan && nxc <= 32 && nxc < M) {
-            mx = kb[0];
-            for (int x = 0; x < nxc; ++x) mx = fmaxf(mx, kb[M - 1 - x]);
+        if (!any_nan && nxc < 32 && nxc < M) {
+            // lane x < nxc looks at slot M-1-x, the others at the head
+            mx = kb[(tid & 31) < nxc ? M - 1 - (tid & 31) : 0];
+            asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(mx) : "f"(mx));
         } else {
             mx = w[0];
 #pragma unroll
             for (int e = 1; e < E; ++e) mx = fmaxf(mx, w[e]);
             mx = block_max(mx, reinterpret_cast<float*>(ired));
         }
-#pragma unroll
-        for (int e = 0; e < E; ++e) w[e] = pf_expneg(w[e] - mx);
+        pf_expneg_row<E>(w, mx);
     }
     if (D.ess_frac > 0.0f) {
         // effective sample size (sum w)^2 / sum w^2 in FP64; a sub-filter whose

@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(M / E, pf_min_blocks(M / E, pf_k1_warps(Mdl::S
     __shared__ typename Mdl::Consts cst;
     __shared__ double dred[64];
     __shared__ int ired[34];
-    __shared__ float s_lmax;
+    __shared__ float s_max[NT / 32];
     __shared__ uint64_t mbar;
     __shared__ FilterDesc sdesc;
     const FilterDesc& D = load_desc(sdesc, descs);
@@ -131,6 +131,9 @@ __global__ void __launch_bounds__(M / E, pf_min_blocks(M / E, pf_k1_warps(Mdl::S
     }
 
     // ---- S
+    const float lmax = cta_max<NT, E>(okey, s_max);
+    write_partials<Mdl, E, NT, k1_stage_bytes<Mdl, M, true>(), true>(
+        D, b, D.log_weights ? lmax : 0.0f, okey, st, sn, cs, reinterpret_cast<double*>(stage));
     float k[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) k[e] = okey[e];
@@ -138,14 +141,9 @@ __global__ void __launch_bounds__(M / E, pf_min_blocks(M / E, pf_k1_warps(Mdl::S
         k, st, sk, si, stage,
         [&] {
             stv<E>(cur_key + base, k);
-            if (tid == 0) {
-                D.winner[b] = k[0];
-                s_lmax = k[0];
-            }
+            if (tid == 0) D.winner[b] = k[0];
         },
         [&](int v, const float(&o)[E]) { stv<E>(cur_tmp + v * T + base, o); });
-    write_partials<Mdl, E, NT, k1_stage_bytes<Mdl, M, true>()>(D, b, D.log_weights ? s_lmax : 0.0f, okey, st, sn,
-                                                                cs, reinterpret_cast<double*>(stage));
 
     // ---- E (warp 0 wrote the partials)
     if (tid < 32) estimate_last_done<S>(D, X, b, in, step_ctr, tid);
