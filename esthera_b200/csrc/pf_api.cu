@@ -141,7 +141,8 @@ bool pfhost::dependent_launch_pays(int grid, int M, int E, int S, int device)
         }
         sms[device].store(n, std::memory_order_relaxed);
     }
-    return grid > n * pf_min_blocks(M / E, pf_k1_warps(S, E));
+    const int wave = n * pf_min_blocks(M / E, pf_k1_warps(S, E));
+    return S <= 3 || 2 * grid <= wave || grid > wave;
 }
 
 extern "C" pf_status pf_model_info(pf_model_id model, int32_t* S, int32_t* K, int32_t* C, int32_t* Z)
@@ -247,7 +248,9 @@ struct pf_filter {
     pf_step_input* h_in = nullptr;
     int64_t dev_bytes = 0;
     int32_t steps_done = 0;
-    cudaGraphExec_t graph = nullptr;
+    cudaGraphExec_t graph = nullptr;                 // one step
+    cudaGraphExec_t graph_n[2] = {nullptr, nullptr}; // kRunSteps[] steps each
+    int64_t replayed = 0;                            // steps run over the current arrays
     const pf_step_input* graph_inputs = nullptr;
     pf_estimate* graph_est = nullptr;
     int32_t graph_cap = 0;
@@ -274,6 +277,27 @@ struct pf_filter {
     int nphase = 0;
 };
 
+// A run over device arrays replays graphs of 16 and 4 steps -- one launch from
+// the host for all of them, and inside, each sampling kernel a programmatic
+// dependent of the step before's resampling kernel -- and the one-step graph
+// for the rest.  The larger graphs are captured (about 0.1 ms) once the filter
+// has run kRunAfter steps, so that a short run does not pay for them.  One
+// filter, us per step, one-step graphs before -> now: 8 sub-filters of 512
+// (unicycle) 12.8 -> 10.4, 256: 16.0 -> 14.2, 2048: 35.5 -> 33.3; the DH arm's
+// 256 sub-filters of 256 17.1 -> 13.6, 1024: 27.2 -> 24.2 (three such filters
+// at once 18.5 -> 19.4: there the GPU was full before).
+constexpr int kRunSteps[2] = {16, 4};
+constexpr int64_t kRunAfter = 64;
+
+static void drop_graphs(pf_filter* f)
+{
+    for (cudaGraphExec_t* g : {&f->graph, &f->graph_n[0], &f->graph_n[1]}) {
+        if (*g) cudaGraphExecDestroy(*g);
+        *g = nullptr;
+    }
+    f->replayed = 0;
+}
+
 template <class T>
 static pf_status dalloc(pf_filter* f, T** p, size_t count)
 {
@@ -297,7 +321,7 @@ static pf_status dalloc(pf_filter* f, T** p, size_t count)
 static void release(pf_filter* f)
 {
     if (!f) return;
-    if (f->graph) cudaGraphExecDestroy(f->graph);
+    drop_graphs(f);
     if (f->ev_sampled) cudaEventDestroy(f->ev_sampled);
     for (cudaEvent_t e : f->ev)
         if (e) cudaEventDestroy(e);
@@ -717,10 +741,7 @@ extern "C" pf_status pf_record_selection(pf_filter* f, int32_t enable)
         if (s != PF_OK) return s;
     }
     if (!enable) f->sel = nullptr;  // the buffer stays allocated until destroy
-    if (f->graph) {
-        cudaGraphExecDestroy(f->graph);
-        f->graph = nullptr;
-    }
+    drop_graphs(f);
     return upload_descs(f, f->graph_est);
 }
 
@@ -738,8 +759,12 @@ extern "C" pf_status pf_get_selection(pf_filter* f, int32_t* sel)
 
 // The launch sequence of one step on f->stream.  desc: device descriptor to use.
 // With timing on, an event is recorded before the first and after every launch
-// (also inside a captured graph, as event-record nodes).
-static pf_status enqueue_step(pf_filter* f, const FilterDesc* desc, InputRef in, int32_t* ctr_inc)
+// (also inside a captured graph, as event-record nodes).  ctr_inc: the counter
+// that advances by in.inc at the end of the step (null: not in this step).
+// chained: the launch before it in the stream is the resampling kernel of the
+// same filter's step before.
+static pf_status enqueue_step(pf_filter* f, const FilterDesc* desc, InputRef in, int32_t* ctr_inc,
+                              bool chained = false)
 {
     const int M = f->M, E = f->E, N = f->N;
     cudaStream_t st = f->stream;
@@ -772,7 +797,8 @@ static pf_status enqueue_step(pf_filter* f, const FilterDesc* desc, InputRef in,
             CU(mark("a2a_merge"));
         }
     } else if (f->pipe == PF_PIPELINE_SPLIT) {
-        CU(f->ops.sample_sort(M, E, f->tp, c.rng == PF_RNG_SUBFILTER, N, st, desc, nullptr, in));
+        const bool fr = c.rng == PF_RNG_SUBFILTER;
+        CU(f->ops.sample_sort(M, E, f->tp, fr, N, st, desc, nullptr, in, chained && fr));
         CU(mark("sample_sort"));
         if (c.exchange == PF_EXCHANGE_ALL2ALL && f->t > 0) {
             CU(launch_a2a_merge(1, desc, st));
@@ -787,7 +813,7 @@ static pf_status enqueue_step(pf_filter* f, const FilterDesc* desc, InputRef in,
         CU(f->ops.exchange_resample(M, E, c.resampler, N + estimate_ctas(N), st, desc, nullptr, in,
                                     late ? nullptr : ctr_inc, virt));
         CU(mark("exchange_resample"));
-        if (late) CU(launch_counter_inc(ctr_inc, st));
+        if (late) CU(launch_counter_add(ctr_inc, in.inc, st));
     } else {
         CU(f->ops.sample_weight(M, E, N, st, desc, nullptr, in));
         CU(mark("sample_weight"));
@@ -816,10 +842,7 @@ extern "C" pf_status pf_set_timing(pf_filter* f, int32_t enable)
     CU(cudaStreamSynchronize(f->stream));
     if (enable && !f->ev[0])
         for (auto& e : f->ev) CU(cudaEventCreate(&e));
-    if ((enable != 0) != (f->timing != 0) && f->graph) {
-        cudaGraphExecDestroy(f->graph);
-        f->graph = nullptr;
-    }
+    if ((enable != 0) != (f->timing != 0)) drop_graphs(f);
     f->timing = enable ? 1 : 0;
     return PF_OK;
 }
@@ -864,40 +887,73 @@ extern "C" pf_status pf_step(pf_filter* f, const pf_step_input* in, pf_estimate*
     return PF_OK;
 }
 
-// The graph of one step reading inputs[ctr % capacity] and writing
-// estimates[ctr % capacity] (ctr: the filter's device step counter), rebuilt
-// when the arrays change.
-static pf_status ensure_run_graph(pf_filter* f, const pf_step_input* d_inputs, pf_estimate* d_estimates,
-                                  int32_t capacity)
+// The graph of `steps` steps reading inputs[ctr % capacity] and writing
+// estimates[ctr % capacity] (ctr: the filter's device step counter).
+static pf_status capture_run(pf_filter* f, int steps, cudaGraphExec_t* exec)
 {
-    if (f->graph && f->graph_inputs == d_inputs && f->graph_est == d_estimates && f->graph_cap == capacity)
-        return PF_OK;
-    CU(cudaStreamSynchronize(f->stream));
-    if (f->graph) {
-        cudaGraphExecDestroy(f->graph);
-        f->graph = nullptr;
-    }
-    pf_status s = upload_descs(f, d_estimates);
-    if (s != PF_OK) return s;
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(f->stream, cudaStreamCaptureModeThreadLocal));
-    InputRef ir{d_inputs, 0, f->ctr, capacity};
-    s = enqueue_step(f, f->d_desc + 1, ir, f->ctr);
+    pf_status s = PF_OK;
+    for (int i = 0; i < steps && s == PF_OK; ++i) {
+        InputRef ir{f->graph_inputs, 0, f->ctr, f->graph_cap};
+        if (f->pipe == PF_PIPELINE_SPLIT) {
+            // the counter stands still within the graph, so that a sampling
+            // kernel can read it before the step before has ended
+            ir.add = i;
+            ir.inc = steps;
+            s = enqueue_step(f, f->d_desc + 1, ir, i == steps - 1 ? f->ctr : nullptr, i > 0);
+        } else {
+            s = enqueue_step(f, f->d_desc + 1, ir, f->ctr);
+        }
+    }
     cudaError_t e = cudaStreamEndCapture(f->stream, &g);
     if (s != PF_OK) {
         if (g) cudaGraphDestroy(g);
         return s;
     }
     if (e != cudaSuccess) return fail(PF_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&f->graph, g, 0);
+    e = cudaGraphInstantiate(exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
-        f->graph = nullptr;
+        *exec = nullptr;
         return fail(PF_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
     }
+    return PF_OK;
+}
+
+// The one-step graph, rebuilt when the arrays change.
+static pf_status ensure_run_graph(pf_filter* f, const pf_step_input* d_inputs, pf_estimate* d_estimates,
+                                  int32_t capacity)
+{
+    if (f->graph && f->graph_inputs == d_inputs && f->graph_est == d_estimates && f->graph_cap == capacity)
+        return PF_OK;
+    CU(cudaStreamSynchronize(f->stream));
+    drop_graphs(f);
+    pf_status s = upload_descs(f, d_estimates);
+    if (s != PF_OK) return s;
     f->graph_inputs = d_inputs;
     f->graph_est = d_estimates;
     f->graph_cap = capacity;
+    return capture_run(f, 1, &f->graph);
+}
+
+// Launches `steps` steps of the run that ensure_run_graph set up.
+static pf_status launch_run(pf_filter* f, int32_t steps)
+{
+    int left = steps;
+    for (int k = 0; k < 2; ++k) {
+        const int n = kRunSteps[k];
+        if (left < n || f->timing) continue;  // (timing records the events of one step)
+        if (!f->graph_n[k]) {
+            if (f->replayed + left < kRunAfter) continue;
+            pf_status s = capture_run(f, n, &f->graph_n[k]);
+            if (s != PF_OK) return s;
+        }
+        for (; left >= n; left -= n) CU(cudaGraphLaunch(f->graph_n[k], f->stream));
+    }
+    for (; left > 0; --left) CU(cudaGraphLaunch(f->graph, f->stream));
+    f->replayed += steps;
+    f->steps_done += steps;
     return PF_OK;
 }
 
@@ -911,9 +967,7 @@ extern "C" pf_status pf_run_device(pf_filter* f, const pf_step_input* d_inputs, 
     if (s != PF_OK) return s;
     CU(cudaMemsetAsync(f->ctr, 0, sizeof(int32_t), f->stream));
     f->q_active = 0;
-    for (int i = 0; i < steps; ++i) CU(cudaGraphLaunch(f->graph, f->stream));
-    f->steps_done += steps;
-    return PF_OK;
+    return launch_run(f, steps);
 }
 
 static pf_status queue_setup(pf_filter* f)
@@ -1010,9 +1064,7 @@ extern "C" pf_status pf_run_device_continue(pf_filter* f, int32_t steps)
 {
     if (!f || !f->graph) return fail(PF_ERR_INVALID, "no run set up (call pf_run_device first)");
     CU(cudaSetDevice(f->cfg.device));
-    for (int i = 0; i < steps; ++i) CU(cudaGraphLaunch(f->graph, f->stream));
-    f->steps_done += steps;
-    return PF_OK;
+    return launch_run(f, steps);
 }
 
 extern "C" pf_status pf_synchronize(pf_filter* f)
@@ -1432,7 +1484,7 @@ extern "C" pf_status pf_shard_sample(pf_filter* f, const pf_step_input* in)
     *f->h_in = *in;
     CU(cudaMemcpyAsync(f->d_in, f->h_in, sizeof(pf_step_input), cudaMemcpyHostToDevice, f->stream));
     InputRef ir{f->d_in, 0, nullptr, 0, f->steps_done};
-    CU(f->ops.sample_sort(f->M, f->E, f->tp, true, f->N, f->stream, f->d_desc, nullptr, ir));
+    CU(f->ops.sample_sort(f->M, f->E, f->tp, true, f->N, f->stream, f->d_desc, nullptr, ir, false));
     CU(launch_shard_pack(f->d_desc, f->halo_out, f->mi.S, f->dx * f->t, f->stream));
     CU(cudaEventRecord(f->ev_sampled, f->stream));
     return PF_OK;

@@ -187,18 +187,19 @@ static pf_status batch_status(int32_t st)
     return PF_OK;
 }
 
-static pf_status enqueue_batch_step(pf_batch* B, const FilterDesc* desc, InputRef in, int32_t* ctr_inc)
+// chained: the launch before it in the stream is the resampling kernel of the step before
+static pf_status enqueue_batch_step(pf_batch* B, const FilterDesc* desc, InputRef in, bool chained)
 {
     for (const pf_batch::Group& g : B->groups) {
         const int2* map = B->map + g.map_off;  // the estimate CTAs, then the sub-filters
-        CU(B->ops.sample_sort(g.M, g.E, g.TP, true, g.NS, B->stream, desc, map + g.NE, in));
+        CU(B->ops.sample_sort(g.M, g.E, g.TP, true, g.NS, B->stream, desc, map + g.NE, in, chained));
+        chained = true;
         // a programmatic dependent of the sampling kernel when that pays (starts in its last wave, waits for
         // the grid)
         const int virt = dependent_launch_pays(g.NS, g.M, g.E, B->mi.S, B->cfg.device) ? 3 : 1;
         CU(B->ops.exchange_resample(g.M, g.E, B->cfg.resampler, g.NE + g.NS, B->stream, desc, map, in, nullptr,
                                     virt));
     }
-    if (ctr_inc) CU(launch_counter_inc(ctr_inc, B->stream));
     return PF_OK;
 }
 
@@ -454,7 +455,7 @@ extern "C" pf_status pf_batch_step(pf_batch* B, const pf_step_input* inputs, pf_
     memcpy(B->h_in, inputs, sizeof(pf_step_input) * B->F);
     CU(cudaMemcpyAsync(B->d_in, B->h_in, sizeof(pf_step_input) * B->F, cudaMemcpyHostToDevice, B->stream));
     InputRef ir{B->d_in, 1, nullptr, 0, B->steps_done};
-    pf_status s = enqueue_batch_step(B, B->d_desc, ir, nullptr);
+    pf_status s = enqueue_batch_step(B, B->d_desc, ir, false);
     if (s != PF_OK) return s;
     // the estimates and the kernels' status word after them in one copy
     CU(cudaMemcpyAsync(out ? (void*)B->h_est : (void*)(B->h_est + B->F), out ? (void*)B->d_est : (void*)(B->d_est + B->F),
@@ -476,7 +477,12 @@ static pf_status capture(pf_batch* B, int steps, InputRef ir, cudaGraphExec_t* e
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
     pf_status s = PF_OK;
-    for (int i = 0; i < steps && s == PF_OK; ++i) s = enqueue_batch_step(B, B->d_desc + B->F, ir, B->ctr);
+    for (int i = 0; i < steps && s == PF_OK; ++i) {
+        ir.add = i;  // the counter stands still within the graph and advances at its end
+        s = enqueue_batch_step(B, B->d_desc + B->F, ir, i > 0);
+    }
+    if (s == PF_OK && launch_counter_add(B->ctr, steps, B->stream) != cudaSuccess)
+        s = fail(PF_ERR_CUDA, "graph capture: counter");
     cudaError_t e = cudaStreamEndCapture(B->stream, &g);
     if (s != PF_OK) {
         if (g) cudaGraphDestroy(g);

@@ -423,12 +423,12 @@ cudaError_t launch_shard_estimate(const FilterDesc& D, int S, const float* best_
 // every kernel of the step that reads it is enqueued before it.
 __global__ void k_counter_update(int32_t* ctr, int32_t set, int32_t value)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *ctr = set ? value : *ctr + 1;
+    if (threadIdx.x == 0 && blockIdx.x == 0) *ctr = set ? value : *ctr + value;
 }
 
-cudaError_t launch_counter_inc(int32_t* ctr, cudaStream_t st)
+cudaError_t launch_counter_add(int32_t* ctr, int32_t n, cudaStream_t st)
 {
-    k_counter_update<<<1, 32, 0, st>>>(ctr, 0, 0);
+    k_counter_update<<<1, 32, 0, st>>>(ctr, 0, n);
     return cudaGetLastError();
 }
 

@@ -165,7 +165,7 @@ __device__ __forceinline__ void mtgp_load_linear(MtgpLinear<CAP>& s, const uint3
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int i = tid + r * NT;
-        w[r] = i < kMtgpN ? __ldcs(gstate + i) : 0u;
+        w[r] = i < kMtgpN ? __ldcg(gstate + i) : 0u;
     }
     const uint32_t* P = g_mtgp_params + set * 52;
     const uint32_t tb = tid < 16 ? P[4 + tid] : 0u, tt = tid < 16 ? P[36 + tid] : 0u;
@@ -194,11 +194,12 @@ __device__ __forceinline__ void mtgp_load_linear(MtgpLinear<CAP>& s, const uint3
 // nz[k+1] -- RAW: stored as they are (floats in [1,2)) and the caller applies
 // box_muller to each pair (nz[2q], nz[2q+1]) when it reads them: the same
 // normals, with the Box-Muller chains taken out of the barrier-separated
-// rounds.  Words k >= nbm (k < n) go to emit(k, word).  Returns the shift: the
+// rounds.  Words k >= nbm (k < n) go to emit(k, word), after ready() has run
+// once in every thread.  Returns the shift: the
 // stream's next state word i is x[n + i - shift].  Ends with a barrier.
-template <bool RAW, int NT, int CAP, class Emit>
+template <bool RAW, int NT, int CAP, class Ready, class Emit>
 __device__ __forceinline__ int mtgp_generate_linear(MtgpLinear<CAP>& s, int n, int nbm, float* __restrict__ nz,
-                                                    Emit emit)
+                                                    Ready ready, Emit emit)
 {
     constexpr int PR = (kMtgpLanes / 2 + NT - 1) / NT;  // pairs per thread and round
     const int tid = threadIdx.x;
@@ -273,6 +274,7 @@ __device__ __forceinline__ int mtgp_generate_linear(MtgpLinear<CAP>& s, int n, i
             }
             __syncthreads();
         }
+        ready();
         for (; base < n; base += kMtgpLanes) {
             make_room(base);
 #pragma unroll 1

@@ -37,10 +37,14 @@ struct ModelInfo {
 bool model_info(int model, ModelInfo* mi);
 
 // Whether to launch the resampling kernel as a programmatic dependent of the
-// sampling kernel: measured to pay when the sampling grid runs in more than
-// one wave (its CTAs start in the sampling kernel's last wave: 2^20 unicycle
-// particles, 67.0 -> 62.2 us per step) and to cost when it fits in one (2^18
-// DH-arm particles, 49.8 -> 58.3 us).
+// sampling kernel, whose CTAs it then joins on the SMs to wait there.  Small
+// states: always (8 to 2048 sub-filters of 512 unicycle particles, within runs,
+// us per step without -> with: 11.1 -> 10.4, 20.7 -> 14.2 at 256, 22.3 -> 21.4
+// at 768, 33.2 -> 33.3 at 2048).  Larger states: not when the sampling grid
+// takes more than half of one wave but not more than one, where the waiting
+// CTAs crowd out the sampling kernel's (DH arm, sub-filters of 256: 20.5 ->
+// 13.6 at 256, 22.1 -> 21.8 at 512, but 23.0 -> 23.4 at 768 and 24.2 -> 25.4 at
+// 1024; 43.8 -> 43.9 at 2048).
 bool dependent_launch_pays(int grid, int M, int E, int S, int device);
 const float* init_state_of(int model, const ModelParams& mp);
 uint32_t angle_mask_of(int model);
@@ -48,7 +52,7 @@ int angle_count_of(int model);
 
 // Launch dispatch over the model template.
 struct ModelOps {
-    cudaError_t (*sample_sort)(int, int, int, bool, int, cudaStream_t, const FilterDesc*, const int2*, InputRef);
+    cudaError_t (*sample_sort)(int, int, int, bool, int, cudaStream_t, const FilterDesc*, const int2*, InputRef, bool);
     cudaError_t (*sample_weight)(int, int, int, cudaStream_t, const FilterDesc*, const int2*, InputRef);
     cudaError_t (*block_sort)(int, int, int, cudaStream_t, const FilterDesc*, const int2*);
     cudaError_t (*exchange_resample)(int, int, int, int, cudaStream_t, const FilterDesc*, const int2*, InputRef,

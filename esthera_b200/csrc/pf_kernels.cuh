@@ -90,11 +90,16 @@ __device__ __forceinline__ const FilterDesc& load_desc(FilterDesc& sd, const Fil
     return sd;
 }
 
-// Programmatic dependent launch (split pipeline): the sampling kernel lets the
-// resampling kernel's CTAs launch once all of its own CTAs are running, and
-// those wait in wait_prerequisites() -- after their prologue -- until the
-// sampling kernel has completed and its writes are visible.  Both are no-ops
-// for kernels launched without the programmatic attribute.
+// Programmatic dependent launch (split pipeline): a kernel lets the next one's
+// CTAs launch once all of its own CTAs have passed their own wait, and those
+// wait in wait_prerequisites() -- after what they can do without its results
+// -- until it has completed and its writes are visible.  The resampling kernel
+// follows its step's sampling kernel so, and, within a graph of several steps,
+// the sampling kernel the step before's resampling kernel.  Because
+// allow_dependents() comes after wait_prerequisites() everywhere, a running
+// kernel can only meet its direct predecessor: whatever lies further back has
+// completed before it was launched.  Both are no-ops for kernels launched
+// without the programmatic attribute.
 __device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
@@ -145,15 +150,17 @@ struct InputRef {
     const int32_t* ctr;      // device step counter (graph replays) or null
     int32_t cap;             // inputs / estimates per filter: the counter indexes them modulo cap
     int32_t step;            // step number of this step when there is no device counter
+    int32_t add = 0;         // with a counter: this step's offset from it (several steps in one graph) ...
+    int32_t inc = 1;         // ... and what the last of them adds to it
 };
 
 // Step number within the run: the device counter, else the host-given number.
-__device__ __forceinline__ int32_t run_step(const InputRef& in) { return in.ctr ? *in.ctr : in.step; }
+__device__ __forceinline__ int32_t run_step(const InputRef& in) { return in.ctr ? *in.ctr + in.add : in.step; }
 
 __device__ __forceinline__ int64_t step_index(const InputRef& in)
 {
     // unsigned: a counter that wrapped past 2^31 steps still maps into [0, cap)
-    return in.ctr ? (int64_t)((uint32_t)*in.ctr % (uint32_t)(in.cap > 0 ? in.cap : 1)) : 0;
+    return in.ctr ? (int64_t)((uint32_t)(*in.ctr + in.add) % (uint32_t)(in.cap > 0 ? in.cap : 1)) : 0;
 }
 
 
@@ -173,6 +180,24 @@ __device__ __forceinline__ void ldv(const float* __restrict__ p, float (&o)[E])
     } else {
 #pragma unroll
         for (int q = 0; q < E; ++q) o[q] = p[q];
+    }
+}
+// The same past L1 (rows another kernel may just have written).
+template <int E>
+__device__ __forceinline__ void ldv_l2(const float* p, float (&o)[E])
+{
+    if constexpr (E % 4 == 0) {
+#pragma unroll
+        for (int q = 0; q < E; q += 4) {
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(p + q));
+            o[q] = v.x; o[q + 1] = v.y; o[q + 2] = v.z; o[q + 3] = v.w;
+        }
+    } else if constexpr (E == 2) {
+        const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
+        o[0] = v.x; o[1] = v.y;
+    } else {
+#pragma unroll
+        for (int q = 0; q < E; ++q) o[q] = __ldcg(p + q);
     }
 }
 template <int E>
@@ -357,7 +382,6 @@ __global__ void __launch_bounds__(TP * M / E, pf_min_blocks(TP * M / E, pf_k1_wa
     __shared__ FilterDesc sdesc;
     int f, b;
     cta_target(cta_map, f, b);
-    allow_dependents();
     const FilterDesc& D = load_desc(sdesc, descs + f);
     const int tid = threadIdx.x;
     const int vt = tid / TP, h = tid % TP;  // the thread's E particles, its half of them
@@ -380,10 +404,19 @@ __global__ void __launch_bounds__(TP * M / E, pf_min_blocks(TP * M / E, pf_k1_wa
         });
         const int nbm = D.nbm;
         float* ru = D.ru + (int64_t)b * D.ru_stride;
+        // everything up to the first resampling uniform needs only this
+        // sub-filter's stream; the uniforms, the particles and the sorted copy
+        // are shared with the step before's resampling kernel
         const int shift = mtgp_generate_linear<raw_normals<Mdl, E>(), NT>(
-            ms, D.draws, nbm, nz, [&](int k, uint32_t o) { ru[k - nbm] = __uint_as_float(o); });
+            ms, D.draws, nbm, nz,
+            [] {
+                wait_prerequisites();
+                allow_dependents();
+            },
+            [&](int k, uint32_t o) { ru[k - nbm] = __uint_as_float(o); });
         mtgp_store_linear(ms, gst, D.draws, shift);
     } else {
+        allow_dependents();
         if (tid < 32) Mdl::prepare(cst, *input_of(in, f), D.mp, tid);
     }
     __syncthreads();
@@ -392,7 +425,7 @@ __global__ void __launch_bounds__(TP * M / E, pf_min_blocks(TP * M / E, pf_k1_wa
 #pragma unroll
     for (int v = 0; v < S; ++v) {
         float o[E];
-        ldv<E>(D.state + v * T + base, o);
+        ldv_l2<E>(D.state + v * T + base, o);
 #pragma unroll
         for (int e = 0; e < E; ++e) st[e][v] = o[e];
     }
@@ -1003,7 +1036,7 @@ __device__ __forceinline__ void estimate_group(const FilterDesc& D, int g, const
     last = __shfl_sync(kFull, last, 0);
     if (!last) return;
     __threadfence();
-    const int32_t step_no = in.ctr ? *in.ctr + 1 : 0;
+    const int32_t step_no = in.ctr ? *in.ctr + in.add + 1 : 0;
     if constexpr (STAGED) {
         const int wr = (CAP / staged_stride(NV + 2)) & ~31;
         estimate_final_staged<S>(D, lane, ng, NV, D.tmp, D.est[step_index(in)], step_no, smem, wr);
@@ -1013,7 +1046,7 @@ __device__ __forceinline__ void estimate_group(const FilterDesc& D, int g, const
     if (lane == 0) {
         *D.est_ctr = 0;
         __threadfence();
-        if (step_ctr) *step_ctr += 1;
+        if (step_ctr) *step_ctr += in.inc;
     }
 }
 
@@ -1335,6 +1368,7 @@ __global__ void __launch_bounds__(M / E, pf_min_blocks(M / E, pf_k2_warps(S))) k
     const FilterDesc& D = load_desc(sdesc, descs + f);
     const int tid = threadIdx.x;
     wait_prerequisites();
+    allow_dependents();
     if (b < 0) {
         constexpr int cap = (int)(k2_smem<S, M, E, RES>() / 8);  // doubles of dynamic shared memory
         estimate_group<S, cap>(D, -1 - b, in, step_ctr, reinterpret_cast<double*>(smem));

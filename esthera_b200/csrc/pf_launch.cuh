@@ -26,6 +26,25 @@ inline cudaError_t allow_smem(F* fn, size_t bytes)
                                 (int)bytes);
 }
 
+// fn<<<grid, threads, smem, st>>>(args...), as a programmatic dependent of the
+// launch before it when asked to.
+template <class... P, class... A>
+inline cudaError_t launch_maybe_dependent(bool dependent, void (*fn)(P...), int grid, int threads, size_t smem,
+                                          cudaStream_t st, A... args)
+{
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(grid);
+    lc.blockDim = dim3(threads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at;
+    lc.numAttrs = dependent ? 1 : 0;
+    return cudaLaunchKernelEx(&lc, fn, P(args)...);
+}
+
 template <class Mdl>
 struct Launch {
     static constexpr int S = Mdl::S;
@@ -35,9 +54,10 @@ struct Launch {
         for (int a = 0; a < Mdl::NA; ++a) m |= 1u << Mdl::angle_var(a);
         return m;
     }
-    // tp: threads per particle (1, or 2 with fr)
+    // tp: threads per particle (1, or 2 with fr); dependent: a programmatic dependent of the launch before
+    // it, which must be the resampling kernel of the step before (wait_prerequisites)
     static cudaError_t sample_sort(int M, int E, int tp, bool fr, int grid, cudaStream_t st, const FilterDesc* d,
-                                   const int2* map, InputRef in);
+                                   const int2* map, InputRef in, bool dependent);
     static cudaError_t sample_weight(int M, int E, int grid, cudaStream_t st, const FilterDesc* d, const int2* map,
                                      InputRef in);
     static cudaError_t block_sort(int M, int E, int grid, cudaStream_t st, const FilterDesc* d, const int2* map);
@@ -87,7 +107,7 @@ cudaError_t launch_shard_estimate(const FilterDesc& D, int S, const float* best_
 constexpr int kMixedWaitSrcBytes = 32768;  // the source buffer launch_test_bounded_wait_mixed copies
 cudaError_t launch_test_bounded_wait_mixed(const int32_t* limits, int nthreads, const void* src, int32_t* outcome,
                                            int32_t* copied, cudaStream_t st);
-cudaError_t launch_counter_inc(int32_t* ctr, cudaStream_t st);
+cudaError_t launch_counter_add(int32_t* ctr, int32_t n, cudaStream_t st);
 cudaError_t launch_counter_set(int32_t* ctr, int32_t value, cudaStream_t st);
 
 

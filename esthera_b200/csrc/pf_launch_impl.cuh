@@ -10,7 +10,7 @@ namespace pfdev {
 #if defined(PF_PART_K1)
 template <class Mdl>
 cudaError_t Launch<Mdl>::sample_sort(int M, int E, int tp, bool fr, int grid, cudaStream_t st, const FilterDesc* d,
-                                     const int2* map, InputRef in)
+                                     const int2* map, InputRef in, bool dependent)
 {
 #define PF_K1_ONE(m, e, FR, TP)                                                             \
     {                                                                                       \
@@ -18,8 +18,7 @@ cudaError_t Launch<Mdl>::sample_sort(int M, int E, int tp, bool fr, int grid, cu
         constexpr size_t sm = k1_smem<Mdl, m, FR, TP>();                                    \
         cudaError_t r = allow_smem(fn, sm);                                                 \
         if (r != cudaSuccess) return r;                                                     \
-        fn<<<grid, TP * m / e, sm, st>>>(d, map, in);                                       \
-        return cudaGetLastError();                                                          \
+        return launch_maybe_dependent(dependent, fn, grid, TP * m / e, sm, st, d, map, in); \
     }
 #define PF_K1(m, e)                                                                         \
     if (M == m && E == e) {                                                                 \
@@ -46,21 +45,8 @@ cudaError_t Launch<Mdl>::sample_sort(int M, int E, int tp, bool fr, int grid, cu
         constexpr size_t sm = k2_smem<Mdl::S, m, e, RES>();                \
         cudaError_t r = allow_smem(fn, sm);                                \
         if (r != cudaSuccess) return r;                                    \
-        if (virt & 2) { /* programmatic dependent of the sampling kernel */ \
-            cudaLaunchConfig_t lc = {};                                    \
-            lc.gridDim = dim3(grid);                                       \
-            lc.blockDim = dim3(m / e);                                     \
-            lc.dynamicSmemBytes = sm;                                      \
-            lc.stream = st;                                                \
-            cudaLaunchAttribute at[1];                                     \
-            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; \
-            at[0].val.programmaticStreamSerializationAllowed = 1;          \
-            lc.attrs = at;                                                 \
-            lc.numAttrs = 1;                                               \
-            return cudaLaunchKernelEx(&lc, fn, d, map, in, ctr, virt & 1); \
-        }                                                                  \
-        fn<<<grid, m / e, sm, st>>>(d, map, in, ctr, virt & 1);            \
-        return cudaGetLastError();                                         \
+        /* virt & 2: a programmatic dependent of the sampling kernel */     \
+        return launch_maybe_dependent((virt & 2) != 0, fn, grid, m / e, sm, st, d, map, in, ctr, virt & 1); \
     }
 #define PF_K2_CASE_0(m, e) PF_K2_CASE(m, e, 0)
 #define PF_K2_CASE_1(m, e) PF_K2_CASE(m, e, 1)

@@ -574,7 +574,7 @@ extern "C" pf_status pf_server_launch(pf_server* s, int32_t* n_launched)
         const ModelOps ops = model_ops(m);
         const int E = s->E[m];
         InputRef ir{s->d_slot_in, 1, nullptr, 0, 0};
-        CU(ops.sample_sort(M, E, 1, true, (int)ctas[m], ms, s->d_desc, s->d_map[m] + ests[m], ir));
+        CU(ops.sample_sort(M, E, 1, true, (int)ctas[m], ms, s->d_desc, s->d_map[m] + ests[m], ir, false));
         ModelInfo mi;
         model_info(m, &mi);
         const int virt = dependent_launch_pays((int)ctas[m], M, E, mi.S, s->device) ? 3 : 1;

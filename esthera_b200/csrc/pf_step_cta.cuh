@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(M / E, pf_min_blocks(M / E, pf_k1_warps(Mdl::S
         mtgp_load_linear<NT>(ms, gst, (D.stream_base + b) % kMtgpSets, D.mask, [] {});
         const int nbm = D.nbm;
         const int shift = mtgp_generate_linear<raw_normals<Mdl, E>(), NT>(
-            ms, D.draws, nbm, nz, [&](int k, uint32_t o) { ru[k - nbm] = __uint_as_float(o); });
+            ms, D.draws, nbm, nz, [] {}, [&](int k, uint32_t o) { ru[k - nbm] = __uint_as_float(o); });
         mtgp_store_linear(ms, gst, D.draws, shift);
     }
     __syncthreads();
