@@ -1,11 +1,12 @@
 // pf_estimate.cu -- posterior estimate of a set of particles as a kernel-level
-// entry point: FP64 partial sums of the sub-filters into a scratch array in
-// global memory (k_est_partials, a warp or a CTA per sub-filter, one row per
-// CTA), then one CTA combining the rows with log-sum-exp rescaling.  The same
-// arithmetic as the filter's own estimate: weights exp(key - max) in FP32 with
-// the sub-filter's maximum, sums in FP64, circular means for angular variables,
+// entry point: FP64 partial sums of the sub-filters (one to sixteen warps each)
+// into a scratch array in global memory, one row per CTA, and the last CTA to
+// finish combining the rows with log-sum-exp rescaling.  The same arithmetic
+// as the filter's own estimate: weights exp(key - max) in FP32 with the
+// sub-filter's maximum, sums in FP64, circular means for angular variables,
 // the reference's winner (first maximum key, thrust::max_element semantics,
 // src/partfilt/cuda/pf_generic_soa.cu:1014-1017).
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -21,7 +22,14 @@ constexpr int kEstMaxState = 16;
 // winner's key, [2] its particle index (-1: every key is NaN), [3] sum w,
 // [4+v] sum w x_v (angles: sum w sin x_v), [4+S+a] sum w cos of the a-th angle.
 constexpr int kEstStride = 4 + 2 * kEstMaxState;
-constexpr int kEstFinalThreads = 512;
+constexpr int kEstThreads = 512, kEstWarps = kEstThreads / 32;
+
+// Tickets of the CTAs that have written their row, one per call in turn (a
+// call's last CTA sets its own back to 0), so that calls overlapping on the GPU
+// do not count each other's CTAs.
+constexpr int kEstTickets = 256;
+static __device__ unsigned g_est_tickets[kEstTickets];
+static std::atomic<unsigned> g_est_calls{0};
 
 // V consecutive floats (V = 4: one 16-byte load).
 template <int V>
@@ -35,27 +43,121 @@ __device__ __forceinline__ void est_load(const float* __restrict__ p, float (&o)
     }
 }
 
-// Partial sums of the sub-filters, TW warps each (TW = 1: the CTA's four warps
-// take four sub-filters; TW = 8: the CTA's eight warps share one), combined in
-// shared memory into one row per CTA.  V = 4 reads four particles a lane and
-// load, for rows that are 16-byte aligned.
+// The rows part[0 .. nrow) into one pf_estimate, one CTA.  Thread r weighs row
+// r, then each warp adds every 16th row, lane j its value j (a row is one
+// coalesced read), in windows of 512 rows.
+__device__ void est_final(const double* part, const float* __restrict__ keys, const float* __restrict__ state, int S,
+                          int64_t T, int m, int nrow, uint32_t angle_mask, int log_weights,
+                          pf_estimate* __restrict__ out, double (*red)[kEstStride])
+{
+    __shared__ double scale[kEstThreads];
+    __shared__ double sum[kEstStride];
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    double gm = -INFINITY, bk = -INFINITY, bi = -1.0;
+    auto offer = [&](double ok, double oi) {
+        if (oi >= 0.0 && (bi < 0.0 || ok > bk || (ok == bk && oi < bi))) {
+            bk = ok;
+            bi = oi;
+        }
+    };
+    for (int r = tid; r < nrow; r += kEstThreads) {
+        const double* p = part + (int64_t)r * kEstStride;
+        gm = fmax(gm, __ldcg(p));
+        offer(__ldcg(p + 1), __ldcg(p + 2));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        gm = fmax(gm, __shfl_xor_sync(kFull, gm, o));
+        const double ok = __shfl_xor_sync(kFull, bk, o);
+        const double oi = __shfl_xor_sync(kFull, bi, o);
+        offer(ok, oi);
+    }
+    if (lane == 0) {
+        red[wp][0] = gm;
+        red[wp][1] = bk;
+        red[wp][2] = bi;
+    }
+    __syncthreads();
+    for (int w = 0; w < kEstWarps; ++w) {
+        gm = fmax(gm, red[w][0]);
+        offer(red[w][1], red[w][2]);
+    }
+    if (!log_weights) gm = 0.0;
+    const int nv = 1 + S + __popc(angle_mask & ((1u << S) - 1u));
+    double a0 = 0.0, a1 = 0.0;  // values lane and lane + 32
+    for (int r0 = 0; r0 < nrow; r0 += kEstThreads) {
+        const int nr = min(kEstThreads, nrow - r0);
+        __syncthreads();
+        if (tid < nr) scale[tid] = log_weights ? exp(__ldcg(part + (int64_t)(r0 + tid) * kEstStride) - gm) : 1.0;
+        __syncthreads();
+        const double* p = part + (int64_t)r0 * kEstStride + 3 + lane;
+        if (lane < nv) {
+#pragma unroll 8
+            for (int r = wp; r < nr; r += kEstWarps) a0 += scale[r] * __ldcg(p + (int64_t)r * kEstStride);
+        }
+        if (lane + 32 < nv)
+            for (int r = wp; r < nr; r += kEstWarps) a1 += scale[r] * __ldcg(p + 32 + (int64_t)r * kEstStride);
+    }
+    __syncthreads();
+    red[wp][lane] = a0;
+    if (lane + 32 < nv) red[wp][lane + 32] = a1;
+    __syncthreads();
+    if (wp != 0) return;
+    for (int j = lane; j < nv; j += 32) {
+        double s = red[0][j];
+        for (int w = 1; w < kEstWarps; ++w) s += red[w][j];
+        sum[j] = s;
+    }
+    __syncwarp();
+    const double W = sum[0];
+    const int64_t best = bi >= 0.0 && (int64_t)bi < T ? (int64_t)bi : 0;
+    if (lane < kEstMaxState) {
+        const int v = lane;
+        double mean = 0.0;
+        float bv = 0.0f;
+        if (v < S) {
+            if ((angle_mask >> v) & 1u) {
+                const int c = __popc(angle_mask & ((1u << v) - 1u));
+                mean = atan2(sum[1 + v], sum[1 + S + c]);
+            } else {
+                mean = sum[1 + v] / W;
+            }
+            bv = state[(int64_t)v * T + best];
+        }
+        out->mean[v] = mean;
+        out->best[v] = bv;
+    }
+    if (lane == 0) {
+        out->log_norm = gm + log(W);
+        out->best_key = keys[best];
+        out->best_subfilter = (int32_t)(best / m);
+        out->step = 0;
+        out->flags = (isfinite(gm) && isfinite(W) && W > 0.0) ? 0 : 1;
+    }
+}
+
+// The sub-filters' sums, TW warps each (a CTA's sixteen warps take 16 / TW
+// sub-filters), combined in shared memory into one row per CTA; the last CTA
+// to write its row (ticket) forms the estimate.  V = 4 reads four particles a
+// lane and load, for rows that are 16-byte aligned.
 //
 // Bound: reading 4 (1 + S) bytes per particle.  The first R loads of the keys
 // -- and, for states of up to 4 variables, of every state row -- are issued
 // before the maximum is reduced, so a sub-filter costs one round trip to
 // memory, and a lane keeps its own sums only for the variables there are.  2^20
-// particles of 3 variables, 2048 sub-filters of 512: 10.6 us (cold) against 59.0 us for one
-// 256-thread CTA per sub-filter with 33 sums per thread whatever S was.
+// particles of 3 variables, 2048 sub-filters of 512: 14.4 us a call, against
+// 16.4 us with the rows combined by a second kernel and 63.2 us for one 256-thread
+// CTA per sub-filter with 33 sums per thread whatever S was.
 template <int S, int TW, int V>
-__global__ void __launch_bounds__(TW == 1 ? 128 : 256)
-    k_est_partials(const float* __restrict__ keys, const float* __restrict__ state, int64_t T, int m, int nsub,
-                   uint32_t angle_mask, int log_weights, double* __restrict__ part)
+__global__ void __launch_bounds__(kEstThreads)
+    k_estimate(const float* __restrict__ keys, const float* __restrict__ state, int64_t T, int m, int nsub,
+               uint32_t angle_mask, int log_weights, double* part, unsigned* ticket, pf_estimate* __restrict__ out)
 {
-    constexpr int NW = TW == 1 ? 4 : 8;          // warps in the CTA
+    constexpr int NW = kEstWarps;
     constexpr int R = V == 4 ? 4 : 8;            // loads of the keys held in registers
     constexpr bool PRE = S <= 4 && V == 4;       // and of the state rows
     __shared__ double red[NW][kEstStride];
-    allow_dependents();
+    __shared__ bool s_last;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     const int wt = wp % TW;                      // warp within the sub-filter's team
     const int b = blockIdx.x * (NW / TW) + wp / TW;
@@ -112,7 +214,7 @@ __global__ void __launch_bounds__(TW == 1 ? 128 : 256)
             ri[wp] = bi;
         }
         __syncthreads();
-        for (int w = 0; w < NW; ++w) offer(rk[w], ri[w]);
+        for (int w = wp - wt; w < wp - wt + TW; ++w) offer(rk[w], ri[w]);
     }
     const float lmax = log_weights ? bk : 0.0f;
     double sw = 0.0, ss[S], sc[S];
@@ -187,17 +289,20 @@ __global__ void __launch_bounds__(TW == 1 ? 128 : 256)
     }
     __syncthreads();
     // one row: the warps' sums scaled to the CTA's maximum (a team's warps have the same one)
-    double* out = part + (int64_t)blockIdx.x * kEstStride;
+    double* row = part + (int64_t)blockIdx.x * kEstStride;
     const int nw = min(NW, (nsub - (int)blockIdx.x * (NW / TW)) * TW);  // warps that had a sub-filter
     double cm = red[0][0];
     for (int w = 1; w < nw; ++w) cm = fmax(cm, red[w][0]);
+    __shared__ double scale[NW];
+    if (threadIdx.x < nw) {
+        const double l = red[threadIdx.x][0];
+        scale[threadIdx.x] = log_weights && l != cm ? exp(l - cm) : 1.0;
+    }
+    __syncthreads();
     for (int j = 3 + threadIdx.x; j < 4 + S + a; j += blockDim.x) {
         double s = 0.0;
-        for (int w = 0; w < nw; ++w) {
-            const double l = red[w][0];
-            s += (log_weights && l != cm ? exp(l - cm) : 1.0) * red[w][j];
-        }
-        out[j] = s;
+        for (int w = 0; w < nw; ++w) s += scale[w] * red[w][j];
+        row[j] = s;
     }
     if (threadIdx.x == 0) {
         double wk = -INFINITY, wi = -1.0;
@@ -208,129 +313,54 @@ __global__ void __launch_bounds__(TW == 1 ? 128 : 256)
                 wi = oi;
             }
         }
-        out[0] = cm;
-        out[1] = wk;
-        out[2] = wi;
+        row[0] = cm;
+        row[1] = wk;
+        row[2] = wi;
     }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    if (threadIdx.x == 0) *ticket = 0;
+    __threadfence();
+    est_final(part, keys, state, S, T, m, (int)gridDim.x, angle_mask, log_weights, out, red);
 }
 
-// Combine the rows into one pf_estimate (one CTA; a programmatic dependent of
-// k_est_partials).  Bound: two round trips to L2 and the exponentials between
-// them.  Thread r weighs row r, then each warp adds every 16th row, lane j its
-// value j (a row is one coalesced read), in windows of 512 rows.  512 rows: 13.2 us (cold)
-// against 18.4 us for one thread per row holding all 33 sums.
-__global__ void __launch_bounds__(kEstFinalThreads)
-    k_est_final(const double* __restrict__ part, const float* __restrict__ keys, const float* __restrict__ state,
-                int S, int64_t T, int m, int nrow, uint32_t angle_mask, int log_weights, pf_estimate* __restrict__ out)
+// Warps per sub-filter: sixteen where the CTAs of fewer would not reach every
+// SM twice or a sub-filter is long, four up to 1184 sub-filters (two CTAs per
+// SM), one beyond.
+static int est_warps(int m, int64_t nsub)
 {
-    constexpr int NW = kEstFinalThreads / 32;
-    __shared__ double red[NW][kEstStride];
-    __shared__ double scale[kEstFinalThreads];
-    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    wait_prerequisites();
-    double gm = -INFINITY, bk = -INFINITY, bi = -1.0;
-    auto offer = [&](double ok, double oi) {
-        if (oi >= 0.0 && (bi < 0.0 || ok > bk || (ok == bk && oi < bi))) {
-            bk = ok;
-            bi = oi;
-        }
-    };
-    for (int r = tid; r < nrow; r += kEstFinalThreads) {
-        const double* p = part + (int64_t)r * kEstStride;
-        gm = fmax(gm, __ldcg(p));
-        offer(__ldcg(p + 1), __ldcg(p + 2));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        gm = fmax(gm, __shfl_xor_sync(kFull, gm, o));
-        const double ok = __shfl_xor_sync(kFull, bk, o);
-        const double oi = __shfl_xor_sync(kFull, bi, o);
-        offer(ok, oi);
-    }
-    if (lane == 0) {
-        red[wp][0] = gm;
-        red[wp][1] = bk;
-        red[wp][2] = bi;
-    }
-    __syncthreads();
-    for (int w = 0; w < NW; ++w) {
-        gm = fmax(gm, red[w][0]);
-        offer(red[w][1], red[w][2]);
-    }
-    if (!log_weights) gm = 0.0;
-    const int nv = 1 + S + __popc(angle_mask & ((1u << S) - 1u));
-    double a0 = 0.0, a1 = 0.0;  // values lane and lane + 32
-    for (int r0 = 0; r0 < nrow; r0 += kEstFinalThreads) {
-        const int nr = min(kEstFinalThreads, nrow - r0);
-        __syncthreads();
-        if (tid < nr) scale[tid] = log_weights ? exp(__ldcg(part + (int64_t)(r0 + tid) * kEstStride) - gm) : 1.0;
-        __syncthreads();
-        const double* p = part + (int64_t)r0 * kEstStride + 3 + lane;
-        if (lane < nv) {
-#pragma unroll 8
-            for (int r = wp; r < nr; r += NW) a0 += scale[r] * __ldcg(p + (int64_t)r * kEstStride);
-        }
-        if (lane + 32 < nv)
-            for (int r = wp; r < nr; r += NW) a1 += scale[r] * __ldcg(p + 32 + (int64_t)r * kEstStride);
-    }
-    __syncthreads();
-    red[wp][lane] = a0;
-    if (lane + 32 < nv) red[wp][lane + 32] = a1;
-    __syncthreads();
-    if (wp != 0) return;
-    __shared__ double sum[kEstStride];
-    for (int j = lane; j < nv; j += 32) {
-        double s = red[0][j];
-        for (int w = 1; w < NW; ++w) s += red[w][j];
-        sum[j] = s;
-    }
-    __syncwarp();
-    const double W = sum[0];
-    const int64_t best = bi >= 0.0 && (int64_t)bi < T ? (int64_t)bi : 0;
-    if (lane < kEstMaxState) {
-        const int v = lane;
-        double mean = 0.0;
-        float bv = 0.0f;
-        if (v < S) {
-            if ((angle_mask >> v) & 1u) {
-                const int c = __popc(angle_mask & ((1u << v) - 1u));
-                mean = atan2(sum[1 + v], sum[1 + S + c]);
-            } else {
-                mean = sum[1 + v] / W;
-            }
-            bv = state[(int64_t)v * T + best];
-        }
-        out->mean[v] = mean;
-        out->best[v] = bv;
-    }
-    if (lane == 0) {
-        out->log_norm = gm + log(W);
-        out->best_key = keys[best];
-        out->best_subfilter = (int32_t)(best / m);
-        out->step = 0;
-        out->flags = (isfinite(gm) && isfinite(W) && W > 0.0) ? 0 : 1;
-    }
+    if (nsub <= 296 || m > 4096) return 16;
+    return nsub <= 1184 || m > 1024 ? 4 : 1;
 }
-
-// A CTA of eight warps per sub-filter where there are too few sub-filters to
-// fill the GPU with one warp each (four to an SM: 592), or where a sub-filter is
-// longer than two rounds of a warp's loads.
-static bool est_team(int m, int64_t nsub) { return m > 1024 || nsub < 592; }
-static int64_t est_rows(int m, int64_t nsub) { return est_team(m, nsub) ? nsub : (nsub + 3) / 4; }
+static int64_t est_rows(int m, int64_t nsub)
+{
+    const int per = kEstWarps / est_warps(m, nsub);
+    return (nsub + per - 1) / per;
+}
 
 template <int S>
-static cudaError_t launch_est_partials(const float* keys, const float* state, int64_t T, int m, int nsub,
-                                       uint32_t angle_mask, int log_weights, double* scratch, cudaStream_t st)
+static cudaError_t launch_est(const float* keys, const float* state, int64_t T, int m, int nsub, uint32_t angle_mask,
+                              int log_weights, double* scratch, unsigned* ticket, pf_estimate* out, cudaStream_t st)
 {
     const bool vec = ((reinterpret_cast<uintptr_t>(keys) | reinterpret_cast<uintptr_t>(state)) & 15) == 0 &&
                      m % 4 == 0 && T % 4 == 0;
     const int rows = (int)est_rows(m, nsub);
-#define PF_EST(TW, V) \
-    k_est_partials<S, TW, V><<<rows, TW == 1 ? 128 : 256, 0, st>>>(keys, state, T, m, nsub, angle_mask, log_weights, scratch)
-    if (est_team(m, nsub)) {
-        if (vec) PF_EST(8, 4);
-        else PF_EST(8, 1);
-    } else {
+#define PF_EST(TW, V)                                                                                        \
+    k_estimate<S, TW, V><<<rows, kEstThreads, 0, st>>>(keys, state, T, m, nsub, angle_mask, log_weights, scratch, \
+                                                       ticket, out)
+    switch (est_warps(m, nsub)) {
+    case 16:
+        if (vec) PF_EST(16, 4);
+        else PF_EST(16, 1);
+        break;
+    case 4:
+        if (vec) PF_EST(4, 4);
+        else PF_EST(4, 1);
+        break;
+    default:
         if (vec) PF_EST(1, 4);
         else PF_EST(1, 1);
     }
@@ -338,32 +368,22 @@ static cudaError_t launch_est_partials(const float* keys, const float* state, in
     return cudaGetLastError();
 }
 
-// Validates the shape and launches partials + final on `st` with the given scratch.
+// Launches the estimate on `st` with the given scratch (tickets: the device
+// address of g_est_tickets).
 static cudaError_t launch_estimate(const float* keys, const float* state, int S, int64_t T, int m,
-                                   uint32_t angle_mask, int log_weights, double* scratch, pf_estimate* out,
-                                   cudaStream_t st)
+                                   uint32_t angle_mask, int log_weights, double* scratch, unsigned* tickets,
+                                   pf_estimate* out, cudaStream_t st)
 {
     const int nsub = (int)(T / m);
-    cudaError_t e = cudaErrorInvalidValue;
+    unsigned* t = tickets + g_est_calls.fetch_add(1u, std::memory_order_relaxed) % kEstTickets;
     switch (S) {
 #define PF_EST_S(s) \
-    case s: e = launch_est_partials<s>(keys, state, T, m, nsub, angle_mask, log_weights, scratch, st); break;
+    case s: return launch_est<s>(keys, state, T, m, nsub, angle_mask, log_weights, scratch, t, out, st);
         PF_EST_S(1) PF_EST_S(2) PF_EST_S(3) PF_EST_S(4) PF_EST_S(5) PF_EST_S(6) PF_EST_S(7) PF_EST_S(8)
         PF_EST_S(9) PF_EST_S(10) PF_EST_S(11) PF_EST_S(12) PF_EST_S(13) PF_EST_S(14) PF_EST_S(15) PF_EST_S(16)
 #undef PF_EST_S
     }
-    if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(1);
-    lc.blockDim = dim3(kEstFinalThreads);
-    lc.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    return cudaLaunchKernelEx(&lc, k_est_final, (const double*)scratch, keys, state, S, T, m,
-                              (int)est_rows(m, nsub), angle_mask, log_weights, out);
+    return cudaErrorInvalidValue;
 }
 
 static bool estimate_shape_ok(int S, int64_t T, int m, std::string* why)
@@ -412,7 +432,10 @@ extern "C" pf_status pfk_estimate(const float* keys, const float* state, int32_t
     if (e == cudaSuccess) e = cudaMalloc(&de, sizeof(pf_estimate));
     if (e == cudaSuccess) e = cudaMemcpy(dk, keys, (size_t)T * 4, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(ds, state, (size_t)T * num_state * 4, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = launch_estimate(dk, ds, num_state, T, m, angle_mask, log_weights, dp, de, 0);
+    void* tickets = nullptr;
+    if (e == cudaSuccess) e = cudaGetSymbolAddress(&tickets, g_est_tickets);
+    if (e == cudaSuccess)
+        e = launch_estimate(dk, ds, num_state, T, m, angle_mask, log_weights, dp, static_cast<unsigned*>(tickets), de, 0);
     if (e == cudaSuccess) e = cudaMemcpy(out, de, sizeof(pf_estimate), cudaMemcpyDeviceToHost);
     cudaFree(dk);
     cudaFree(ds);
@@ -438,12 +461,13 @@ constexpr int kNoAllocMaxSubfilters = 4096;  // 4096 * 36 doubles = 1.18 MB per 
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocMaxSubfilters * kEstStride];
 
 static std::mutex g_noalloc_mu;
-// Device address of g_noalloc_scratch per device ordinal, valid for the CUDA
+// Device addresses of g_noalloc_scratch and g_est_tickets per device ordinal, valid for the CUDA
 // context whose process-unique id is stored beside it: cudaDeviceReset (or a
 // caller switching to another context on the same ordinal) loads the module
 // afresh, possibly at another address, and the new context has a new id, so
 // the next call looks the address up again instead of using a stale one.
 static double* g_noalloc_ptr[256];
+static unsigned* g_noalloc_tickets[256];
 static unsigned long long g_noalloc_ctx[256];
 
 // The current context's process-unique id (cuCtxGetId; ids are never reused
@@ -491,6 +515,7 @@ extern "C" pf_status pfk_estimate_noalloc(const float* d_keys, const float* d_st
         return pfi_fail(PF_ERR_CUDA, "no current CUDA device");
     }
     double* scratch = nullptr;
+    unsigned* tickets = nullptr;
     {
         // Once per device (and again after the device's context was replaced),
         // with that device current: the host-side name of the array is only a
@@ -500,16 +525,20 @@ extern "C" pf_status pfk_estimate_noalloc(const float* d_keys, const float* d_st
         if (!g_noalloc_ptr[dev] || !ctx || ctx != g_noalloc_ctx[dev]) {
             void* p = nullptr;
             e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-            if (e != cudaSuccess || !p) {
+            void* q = nullptr;
+            if (e == cudaSuccess) e = cudaGetSymbolAddress(&q, g_est_tickets);
+            if (e != cudaSuccess || !p || !q) {
                 cudaGetLastError();
                 return pfi_fail(PF_ERR_CUDA, "cudaGetSymbolAddress of the static scratch failed");
             }
+            g_noalloc_tickets[dev] = static_cast<unsigned*>(q);
             g_noalloc_ptr[dev] = static_cast<double*>(p);
             g_noalloc_ctx[dev] = current_context_id();  // the lookup made the context current if none was
         }
         scratch = g_noalloc_ptr[dev];
+        tickets = g_noalloc_tickets[dev];
     }
-    e = launch_estimate(d_keys, d_state, num_state, num_particles, m, angle_mask, log_weights, scratch, d_out,
+    e = launch_estimate(d_keys, d_state, num_state, num_particles, m, angle_mask, log_weights, scratch, tickets, d_out,
                         static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) {
         cudaGetLastError();
