@@ -240,12 +240,9 @@ struct pf_filter {
     uint32_t* mtgp = nullptr;
     int32_t *a2a = nullptr, *sel = nullptr, *ctr = nullptr, *est_ctr = nullptr;
     double* gpart = nullptr;
-    pf_estimate* d_est = nullptr;
-    pf_step_input* d_in = nullptr;
-    FilterDesc* d_desc = nullptr;  // [0]: pf_step, [1]: pf_run_device
+    FilterDesc* d_desc = nullptr;  // [0]: pf_step, [1]: pf_run_device, [2]: pf_step_submit
     FilterDesc h_desc;
-    pf_estimate* h_est = nullptr;
-    pf_step_input* h_in = nullptr;
+    pf_estimate* h_est = nullptr;  // pinned, written by the kernels: [0] pf_step's estimate, then the status word
     int64_t dev_bytes = 0;
     int32_t steps_done = 0;
     cudaGraphExec_t graph = nullptr;                 // one step
@@ -254,13 +251,11 @@ struct pf_filter {
     const pf_step_input* graph_inputs = nullptr;
     pf_estimate* graph_est = nullptr;
     int32_t graph_cap = 0;
-    // submit / collect queue (pf_step_submit): pinned and device rings of
-    // inputs and estimates, an upload and a download stream, events per slot
-    pf_step_input *h_q_in = nullptr, *d_q_in = nullptr;
-    pf_estimate *h_q_est = nullptr, *d_q_est = nullptr;
-    cudaStream_t q_up = nullptr, q_down = nullptr;
-    cudaEvent_t q_ev_up[PF_QUEUE_DEPTH] = {}, q_ev_done[PF_QUEUE_DEPTH] = {}, q_ev_got[PF_QUEUE_DEPTH] = {};
-    int q_active = 0;   // the device counter holds q_next (else set it before the next submit)
+    // submit / collect queue (pf_step_submit): a pinned ring of estimates that
+    // the kernels write, and of the words that say an estimate is there
+    pf_estimate* h_q_est = nullptr;
+    int32_t* h_q_done = nullptr;
+    int q_active = 0;   // the last step of the stream is step q_next - 1, submitted here
     int q_pending = 0;  // submitted, not yet collected
     int32_t q_next = 0; // step number (and slot, modulo the depth) of the next submit
     // a shard of a larger filter (pf_shard_*): global sub-filters b0 ..
@@ -325,18 +320,9 @@ static void release(pf_filter* f)
     if (f->ev_sampled) cudaEventDestroy(f->ev_sampled);
     for (cudaEvent_t e : f->ev)
         if (e) cudaEventDestroy(e);
-    for (int i = 0; i < PF_QUEUE_DEPTH; ++i) {
-        if (f->q_ev_up[i]) cudaEventDestroy(f->q_ev_up[i]);
-        if (f->q_ev_done[i]) cudaEventDestroy(f->q_ev_done[i]);
-        if (f->q_ev_got[i]) cudaEventDestroy(f->q_ev_got[i]);
-    }
-    if (f->q_up) cudaStreamDestroy(f->q_up);
-    if (f->q_down) cudaStreamDestroy(f->q_down);
-    if (f->h_q_in) cudaFreeHost(f->h_q_in);
     if (f->h_q_est) cudaFreeHost(f->h_q_est);
     for (void* p : f->allocs) cudaFree(p);
     if (f->h_est) cudaFreeHost(f->h_est);
-    if (f->h_in) cudaFreeHost(f->h_in);
     if (f->stream) cudaStreamDestroy(f->stream);
     delete f;
 }
@@ -434,9 +420,9 @@ static pf_status validate(const pf_config* c, int model, const ModelInfo& mi, in
     return PF_OK;
 }
 
-// The kernels' status word (PF_STATUS_* bits), stored right after the
-// estimate so that pf_step's estimate copy brings it along.
-static int32_t* status_word(pf_filter* f) { return reinterpret_cast<int32_t*>(f->d_est + 1); }
+// The kernels' status word (PF_STATUS_* bits), in the pinned memory after
+// pf_step's estimate.
+static int32_t* status_word(pf_filter* f) { return reinterpret_cast<int32_t*>(f->h_est + 1); }
 
 static pf_status check_status(int32_t st)
 {
@@ -499,9 +485,10 @@ static void fill_desc(pf_filter* f, FilterDesc& D, pf_estimate* est)
 
 static pf_status upload_descs(pf_filter* f, pf_estimate* run_est)
 {
-    FilterDesc d[2];
-    fill_desc(f, d[0], f->d_est);
+    FilterDesc d[3];
+    fill_desc(f, d[0], f->h_est);
     fill_desc(f, d[1], run_est);
+    fill_desc(f, d[2], f->h_q_est);
     f->h_desc = d[0];
     CU(cudaMemcpyAsync(f->d_desc, d, sizeof(d), cudaMemcpyHostToDevice, f->stream));
     CU(cudaStreamSynchronize(f->stream));
@@ -625,18 +612,15 @@ extern "C" pf_status pf_create(const pf_config* cfg, pf_model_id model, const vo
     TRY(dalloc(f, &f->ctr, 1));
     TRY(dalloc(f, &f->est_ctr, 1));
     TRY(dalloc(f, &f->gpart, (size_t)((f->N + 31) / 32) * kPartStride));
-    TRY(dalloc(f, &f->d_est, 2));  // [0] the estimate, then the kernels' status word
-    TRY(dalloc(f, &f->d_in, 1));
-    TRY(dalloc(f, &f->d_desc, 2));
-    if (cudaMallocHost(&f->h_est, 2 * sizeof(pf_estimate)) != cudaSuccess ||
-        cudaMallocHost(&f->h_in, sizeof(pf_step_input)) != cudaSuccess) {
+    TRY(dalloc(f, &f->d_desc, 3));
+    if (cudaMallocHost(&f->h_est, 2 * sizeof(pf_estimate)) != cudaSuccess) {
         cudaGetLastError();
         release(f);
         return fail(PF_ERR_NOMEM, "cudaMallocHost failed");
     }
     TRY(init_streams(f));
-    if (cudaMemset(f->est_ctr, 0, 4) != cudaSuccess || cudaMemset(f->ctr, 0, 4) != cudaSuccess ||
-        cudaMemset(f->d_est, 0, 2 * sizeof(pf_estimate)) != cudaSuccess) {
+    memset(f->h_est, 0, 2 * sizeof(pf_estimate));
+    if (cudaMemset(f->est_ctr, 0, 4) != cudaSuccess || cudaMemset(f->ctr, 0, 4) != cudaSuccess) {
         cudaGetLastError();
         release(f);
         return fail(PF_ERR_CUDA, "cudaMemset failed");
@@ -864,21 +848,28 @@ extern "C" const char* pf_phase_name(pf_filter* f, int32_t i)
     return f->phase[i];
 }
 
+// This step's input as kernel parameters.
+static InputRef host_input(const pf_filter* f, const pf_step_input& in)
+{
+    InputRef ir{nullptr, 0, nullptr, 0, f->steps_done};
+    ir.inlined = 1;
+    ir.input = in;
+    return ir;
+}
+
 extern "C" pf_status pf_step(pf_filter* f, const pf_step_input* in, pf_estimate* out)
 {
     if (!f || !in) return fail(PF_ERR_INVALID, "null argument");
     if (f->shard) return fail(PF_ERR_INVALID, "a shard steps through pf_shard_sample / pf_shard_resample");
     CU(cudaSetDevice(f->cfg.device));
-    *f->h_in = *in;
-    CU(cudaMemcpyAsync(f->d_in, f->h_in, sizeof(pf_step_input), cudaMemcpyHostToDevice, f->stream));
-    InputRef ir{f->d_in, 0, nullptr, 0, f->steps_done};
+    // the input travels with the launches and the estimate is written to pinned
+    // host memory: no copy on either side of the kernels
+    InputRef ir = host_input(f, *in);
     pf_status s = enqueue_step(f, f->d_desc, ir, nullptr);
     if (s != PF_OK) return s;
-    CU(cudaMemcpyAsync(f->h_est, f->d_est, sizeof(pf_estimate) + sizeof(int32_t), cudaMemcpyDeviceToHost,
-                       f->stream));
     CU(cudaStreamSynchronize(f->stream));
     f->steps_done++;
-    s = check_status(*reinterpret_cast<const int32_t*>(f->h_est + 1));
+    s = check_status(*status_word(f));
     if (s != PF_OK) return s;
     if (out) {
         *out = *f->h_est;
@@ -972,32 +963,13 @@ extern "C" pf_status pf_run_device(pf_filter* f, const pf_step_input* d_inputs, 
 
 static pf_status queue_setup(pf_filter* f)
 {
-    if (f->d_q_in) return PF_OK;
+    if (f->h_q_est) return PF_OK;
     void* h = nullptr;
-    if (!f->h_q_in) {
-        CU(cudaMallocHost(&h, PF_QUEUE_DEPTH * sizeof(pf_step_input)));
-        f->h_q_in = static_cast<pf_step_input*>(h);
-    }
-    if (!f->h_q_est) {
-        CU(cudaMallocHost(&h, PF_QUEUE_DEPTH * sizeof(pf_estimate)));
-        f->h_q_est = static_cast<pf_estimate*>(h);
-    }
-    if (!f->q_up) CU(cudaStreamCreateWithFlags(&f->q_up, cudaStreamNonBlocking));
-    if (!f->q_down) CU(cudaStreamCreateWithFlags(&f->q_down, cudaStreamNonBlocking));
-    for (int i = 0; i < PF_QUEUE_DEPTH; ++i) {
-        if (!f->q_ev_up[i]) CU(cudaEventCreateWithFlags(&f->q_ev_up[i], cudaEventDisableTiming));
-        if (!f->q_ev_done[i]) CU(cudaEventCreateWithFlags(&f->q_ev_done[i], cudaEventDisableTiming));
-        if (!f->q_ev_got[i]) CU(cudaEventCreateWithFlags(&f->q_ev_got[i], cudaEventDisableTiming));
-    }
-    if (!f->d_q_est) {
-        pf_status s = dalloc(f, &f->d_q_est, PF_QUEUE_DEPTH);
-        if (s != PF_OK) return s;
-    }
-    pf_step_input* di = nullptr;
-    pf_status s = dalloc(f, &di, PF_QUEUE_DEPTH);
-    if (s != PF_OK) return s;
-    f->d_q_in = di;  // set last: marks the queue as set up
-    return PF_OK;
+    CU(cudaMallocHost(&h, PF_QUEUE_DEPTH * (sizeof(pf_estimate) + sizeof(int32_t))));
+    memset(h, 0, PF_QUEUE_DEPTH * (sizeof(pf_estimate) + sizeof(int32_t)));
+    f->h_q_est = static_cast<pf_estimate*>(h);
+    f->h_q_done = reinterpret_cast<int32_t*>(f->h_q_est + PF_QUEUE_DEPTH);
+    return upload_descs(f, f->graph_est);
 }
 
 extern "C" pf_status pf_step_submit(pf_filter* f, const pf_step_input* in)
@@ -1009,27 +981,26 @@ extern "C" pf_status pf_step_submit(pf_filter* f, const pf_step_input* in)
     if (s != PF_OK) return s;
     if (f->q_pending >= PF_QUEUE_DEPTH)
         return fail(PF_ERR_BUSY, "%d steps pending: collect before submitting more", PF_QUEUE_DEPTH);
+    bool chained = f->pipe == PF_PIPELINE_SPLIT && !f->timing;
     if (!f->q_active || f->q_next != f->steps_done) {
         // another call stepped the filter or reset its counter since the last submit
         if (f->q_pending > 0)
             return fail(PF_ERR_BUSY, "collect the pending steps before submitting after another step call");
-        s = ensure_run_graph(f, f->d_q_in, f->d_q_est, PF_QUEUE_DEPTH);
-        if (s != PF_OK) return s;
-        CU(launch_counter_set(f->ctr, f->steps_done, f->stream));
         f->q_next = f->steps_done;
-        f->q_active = 1;
+        chained = false;
     }
-    const int slot = (int)((uint32_t)f->q_next % PF_QUEUE_DEPTH);  // as the device maps its counter
-    f->h_q_in[slot] = *in;
-    CU(cudaMemcpyAsync(f->d_q_in + slot, f->h_q_in + slot, sizeof(pf_step_input), cudaMemcpyHostToDevice, f->q_up));
-    CU(cudaEventRecord(f->q_ev_up[slot], f->q_up));
-    CU(cudaStreamWaitEvent(f->stream, f->q_ev_up[slot], 0));
-    CU(cudaGraphLaunch(f->graph, f->stream));
-    CU(cudaEventRecord(f->q_ev_done[slot], f->stream));
-    CU(cudaStreamWaitEvent(f->q_down, f->q_ev_done[slot], 0));
-    CU(cudaMemcpyAsync(f->h_q_est + slot, f->d_q_est + slot, sizeof(pf_estimate), cudaMemcpyDeviceToHost,
-                       f->q_down));
-    CU(cudaEventRecord(f->q_ev_got[slot], f->q_down));
+    // the step's launches carry the input, follow the step before's as
+    // programmatic dependents, and write the estimate into its pinned slot
+    const int slot = (int)((uint32_t)f->q_next % PF_QUEUE_DEPTH);
+    InputRef ir = host_input(f, *in);
+    ir.slot = slot;
+    ir.done = f->h_q_done + slot;
+    ir.done_value = 1;
+    __atomic_store_n(f->h_q_done + slot, 0, __ATOMIC_RELEASE);
+    f->q_active = 0;  // (until the launches are in the stream)
+    s = enqueue_step(f, f->d_desc + 2, ir, nullptr, chained);
+    if (s != PF_OK) return s;
+    f->q_active = 1;
     f->q_next++;
     f->steps_done++;
     f->q_pending++;
@@ -1045,14 +1016,23 @@ extern "C" pf_status pf_step_collect(pf_filter* f, pf_estimate* out, int32_t max
     while (*count < max && f->q_pending > 0) {
         const int32_t k = f->q_next - f->q_pending;  // oldest pending step
         const int slot = (int)((uint32_t)k % PF_QUEUE_DEPTH);
-        if (wait) {
-            CU(cudaEventSynchronize(f->q_ev_got[slot]));
-        } else {
-            const cudaError_t e = cudaEventQuery(f->q_ev_got[slot]);
-            if (e == cudaErrorNotReady) break;
-            CU(e);
+        auto there = [&] { return __atomic_load_n(f->h_q_done + slot, __ATOMIC_ACQUIRE) != 0; };
+        bool got = there();
+        for (unsigned i = 1; !got && (wait || i == 1); ++i) {
+            // now and then ask the stream: a kernel that failed writes no estimate
+            if (i % 256 == 1) {
+                const cudaError_t e = cudaStreamQuery(f->stream);
+                got = there();
+                if (!got && e == cudaSuccess) return fail(PF_ERR_CUDA, "a submitted step ended without an estimate");
+                if (!got && e != cudaErrorNotReady) CU(e);
+                if (e == cudaErrorNotReady) cudaGetLastError();
+            } else {
+                got = there();
+            }
         }
-        out[(*count)++] = f->h_q_est[slot];
+        if (!got) break;
+        out[*count] = f->h_q_est[slot];
+        out[(*count)++].step = k + 1;
         f->q_pending--;
     }
     return PF_OK;
@@ -1072,9 +1052,7 @@ extern "C" pf_status pf_synchronize(pf_filter* f)
     if (!f) return fail(PF_ERR_INVALID, "null argument");
     CU(cudaSetDevice(f->cfg.device));
     CU(cudaStreamSynchronize(f->stream));
-    int32_t st = 0;
-    CU(cudaMemcpy(&st, status_word(f), sizeof(st), cudaMemcpyDeviceToHost));
-    return check_status(st);
+    return check_status(*status_word(f));
 }
 
 extern "C" void* pf_stream(pf_filter* f) { return f ? (void*)f->stream : nullptr; }
@@ -1481,9 +1459,7 @@ extern "C" pf_status pf_shard_sample(pf_filter* f, const pf_step_input* in)
     TRYS(need_shard(f));
     if (!in) return fail(PF_ERR_INVALID, "null argument");
     CU(cudaSetDevice(f->cfg.device));
-    *f->h_in = *in;
-    CU(cudaMemcpyAsync(f->d_in, f->h_in, sizeof(pf_step_input), cudaMemcpyHostToDevice, f->stream));
-    InputRef ir{f->d_in, 0, nullptr, 0, f->steps_done};
+    InputRef ir = host_input(f, *in);
     CU(f->ops.sample_sort(f->M, f->E, f->tp, true, f->N, f->stream, f->d_desc, nullptr, ir, false));
     CU(launch_shard_pack(f->d_desc, f->halo_out, f->mi.S, f->dx * f->t, f->stream));
     CU(cudaEventRecord(f->ev_sampled, f->stream));
@@ -1542,15 +1518,14 @@ extern "C" pf_status pf_shard_resample(pf_filter* f)
 {
     TRYS(need_shard(f));
     CU(cudaSetDevice(f->cfg.device));
-    InputRef ir{f->d_in, 0, nullptr, 0, f->steps_done};
+    InputRef ir{nullptr, 0, nullptr, 0, f->steps_done};
     CU(f->ops.exchange_resample(f->M, f->E, f->cfg.resampler, f->N + estimate_ctas(f->N), f->stream, f->d_desc,
                                 nullptr, ir, nullptr, 1));
     const int ng = (f->N + 31) / 32;
     CU(launch_shard_rows(f->d_desc, ng, f->rows, f->states, f->mi.S, 2 + f->mi.S + f->na, f->stream));
-    CU(cudaMemcpyAsync(f->h_est, f->d_est, sizeof(pf_estimate) + sizeof(int32_t), cudaMemcpyDeviceToHost, f->stream));
     CU(cudaStreamSynchronize(f->stream));
     f->steps_done++;
-    return check_status(*reinterpret_cast<const int32_t*>(f->h_est + 1));
+    return check_status(*status_word(f));
 }
 
 extern "C" pf_status pf_shard_group_rows(pf_filter* f, double* rows, float* states)

@@ -421,20 +421,14 @@ cudaError_t launch_shard_estimate(const FilterDesc& D, int S, const float* best_
 
 // A run's device step counter, advanced (or set) by a launch of its own once
 // every kernel of the step that reads it is enqueued before it.
-__global__ void k_counter_update(int32_t* ctr, int32_t set, int32_t value)
+__global__ void k_counter_add(int32_t* ctr, int32_t n)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *ctr = set ? value : *ctr + value;
+    if (threadIdx.x == 0 && blockIdx.x == 0) *ctr += n;
 }
 
 cudaError_t launch_counter_add(int32_t* ctr, int32_t n, cudaStream_t st)
 {
-    k_counter_update<<<1, 32, 0, st>>>(ctr, 0, n);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_counter_set(int32_t* ctr, int32_t value, cudaStream_t st)
-{
-    k_counter_update<<<1, 32, 0, st>>>(ctr, 1, value);
+    k_counter_add<<<1, 32, 0, st>>>(ctr, n);
     return cudaGetLastError();
 }
 

@@ -64,7 +64,7 @@ struct FilterDesc {
 // 16-byte aligned (not this library's allocation; the sub-filter kept its
 // propagated particles)
 constexpr int PF_STATUS_WAIT_TIMEOUT = 1;
-constexpr int PF_STATUS_MISALIGNED = 2;
+constexpr int PF_STATUS_MISALIGNED = 0x100;
 
 // Outcome of resample_from: the CTA resampled; it kept its propagated
 // particles (decision uniform, ESS gate, misaligned rows, or a wait that ran
@@ -152,6 +152,14 @@ struct InputRef {
     int32_t step;            // step number of this step when there is no device counter
     int32_t add = 0;         // with a counter: this step's offset from it (several steps in one graph) ...
     int32_t inc = 1;         // ... and what the last of them adds to it
+    // a single filter stepped from the host: the input itself (128 bytes of
+    // kernel parameters instead of a copy ahead of the step), the entry of
+    // est[] that takes the estimate, and where to say that it is there
+    int32_t inlined = 0;
+    int32_t slot = 0;
+    int32_t* done = nullptr;
+    int32_t done_value = 0;
+    pf_step_input input = {};
 };
 
 // Step number within the run: the device counter, else the host-given number.
@@ -160,7 +168,23 @@ __device__ __forceinline__ int32_t run_step(const InputRef& in) { return in.ctr 
 __device__ __forceinline__ int64_t step_index(const InputRef& in)
 {
     // unsigned: a counter that wrapped past 2^31 steps still maps into [0, cap)
-    return in.ctr ? (int64_t)((uint32_t)(*in.ctr + in.add) % (uint32_t)(in.cap > 0 ? in.cap : 1)) : 0;
+    return in.ctr ? (int64_t)((uint32_t)(*in.ctr + in.add) % (uint32_t)(in.cap > 0 ? in.cap : 1)) : in.slot;
+}
+
+// Tells the host that the estimate is written (one lane, after the warp that
+// wrote it has synchronised).
+__device__ __forceinline__ void publish_estimate(const InputRef& in)
+{
+    if (!in.done) return;
+    __threadfence_system();
+    *const_cast<volatile int32_t*>(in.done) = in.done_value;
+}
+
+// A status bit (one byte each, so that no atomic is needed on the pinned host
+// word that a single filter's kernels report to).
+__device__ __forceinline__ void set_status(int32_t* status, int bit)
+{
+    if (status) reinterpret_cast<volatile unsigned char*>(status)[bit == PF_STATUS_WAIT_TIMEOUT ? 0 : 1] = 1;
 }
 
 
@@ -244,7 +268,7 @@ __device__ __forceinline__ int resample_cta(int i, int N)
 
 __device__ __forceinline__ const pf_step_input* input_of(const InputRef& in, int f)
 {
-    return in.base + (int64_t)f * in.filter_stride + step_index(in);
+    return in.inlined ? &in.input : in.base + (int64_t)f * in.filter_stride + step_index(in);
 }
 
 // Whether the sampling kernels leave Box-Muller out of the MTGP32 rounds: for
@@ -372,7 +396,7 @@ __device__ __forceinline__ void write_partials(const FilterDesc& D, int b, float
 // ---------------------------------------------------------------------------
 template <class Mdl, int M, int E, bool FR, int TP = 1>
 __global__ void __launch_bounds__(TP * M / E, pf_min_blocks(TP * M / E, pf_k1_warps(Mdl::S, E) - (TP - 1) * 4)) k_sample_sort(const FilterDesc* __restrict__ descs,
-                                                       const int2* __restrict__ cta_map, InputRef in)
+                                                       const int2* __restrict__ cta_map, const __grid_constant__ InputRef in)
 {
     constexpr int NT = TP * M / E, S = Mdl::S, K = Mdl::K, NA = Mdl::NA;
     constexpr int NANG = NA > 0 ? NA : 1;
@@ -478,7 +502,7 @@ __global__ void __launch_bounds__(TP * M / E, pf_min_blocks(TP * M / E, pf_k1_wa
 // ---------------------------------------------------------------------------
 template <class Mdl, int M, int E>
 __global__ void __launch_bounds__(M / E) k_sample_weight(const FilterDesc* __restrict__ descs,
-                                                         const int2* __restrict__ cta_map, InputRef in)
+                                                         const int2* __restrict__ cta_map, const __grid_constant__ InputRef in)
 {
     constexpr int S = Mdl::S, K = Mdl::K, NA = Mdl::NA;
     constexpr int NANG = NA > 0 ? NA : 1;
@@ -1055,9 +1079,9 @@ __device__ __forceinline__ void estimate_group(const FilterDesc& D, int g, const
         const float best_v = (bv >= 0 && bv < S) ? __ldcg(D.tmp + bv * D.T + (int64_t)best * D.M) : 0.0f;
         estimate_store<S>(D, lane, NV, D.log_weights ? gl : 0.0, won ? wk : -INFINITY, best, best_v, 0.0 + a,
                           D.est[step_index(in)], step_no);
-        if (lane == 0 && step_ctr) {
-            __threadfence();
-            *step_ctr += in.inc;
+        if (lane == 0) {
+            publish_estimate(in);
+            if (step_ctr) *step_ctr += in.inc;
         }
         return;
     }
@@ -1080,6 +1104,7 @@ __device__ __forceinline__ void estimate_group(const FilterDesc& D, int g, const
     }
     if (lane == 0) {
         *D.est_ctr = 0;
+        publish_estimate(in);
         __threadfence();
         if (step_ctr) *step_ctr += in.inc;
     }
@@ -1220,7 +1245,7 @@ __device__ __forceinline__ int resample_from(const FilterDesc& D, int b, const f
         const bool bulk = ((reinterpret_cast<uintptr_t>(src_key) | reinterpret_cast<uintptr_t>(src_tmp) |
                             (uintptr_t)(T * 4)) & 15) == 0;
         if (!bulk) {  // rows not 16-byte aligned: not this library's allocations (no copy issued)
-            if (tid == 0 && D.status) atomicOr(D.status, PF_STATUS_MISALIGNED);
+            if (tid == 0) set_status(D.status, PF_STATUS_MISALIGNED);
             return PF_RS_KEPT;
         }
         if (tid == 0) {
@@ -1241,7 +1266,7 @@ __device__ __forceinline__ int resample_from(const FilterDesc& D, int b, const f
         __syncthreads();  // the mbarrier is initialised
         const int landed = mbar_wait_cta(mbar, 0, kBulkWaitPolls, kBulkDrainPolls);
         if (landed <= 0) {
-            if (tid == 0 && D.status) atomicOr(D.status, PF_STATUS_WAIT_TIMEOUT);
+            if (tid == 0) set_status(D.status, PF_STATUS_WAIT_TIMEOUT);
             return landed < 0 ? PF_RS_LOST : PF_RS_KEPT;
         }
         if (dec_u - 1.0f > D.freq) return PF_RS_KEPT;
@@ -1383,7 +1408,7 @@ __device__ __forceinline__ int resample_from(const FilterDesc& D, int b, const f
 
 template <int S, int M, int E, int RES>
 __global__ void __launch_bounds__(M / E, pf_min_blocks(M / E, pf_k2_warps(S))) k_exchange_resample(const FilterDesc* __restrict__ descs,
-                                                             const int2* __restrict__ cta_map, InputRef in,
+                                                             const int2* __restrict__ cta_map, const __grid_constant__ InputRef in,
                                                              int32_t* step_ctr, int virt)
 {
     extern __shared__ __align__(16) unsigned char smem[];

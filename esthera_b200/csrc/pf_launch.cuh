@@ -108,7 +108,6 @@ constexpr int kMixedWaitSrcBytes = 32768;  // the source buffer launch_test_boun
 cudaError_t launch_test_bounded_wait_mixed(const int32_t* limits, int nthreads, const void* src, int32_t* outcome,
                                            int32_t* copied, cudaStream_t st);
 cudaError_t launch_counter_add(int32_t* ctr, int32_t n, cudaStream_t st);
-cudaError_t launch_counter_set(int32_t* ctr, int32_t value, cudaStream_t st);
 
 
 }  // namespace pfdev

@@ -73,6 +73,7 @@ __device__ __forceinline__ void estimate_last_done(const FilterDesc& D, const St
     const float* cur_tmp = par ? X.tmp2 : D.tmp;
     estimate_write<S>(D, lane, ng, NV, gm, bk, bi, cur_tmp, D.est[step_index(in)], in.ctr ? *in.ctr + 1 : 0);
     if (lane == 0) {
+        publish_estimate(in);
         *D.est_ctr = 0;
         *X.need_init = 0;
         __threadfence();

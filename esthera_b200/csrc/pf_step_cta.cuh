@@ -33,7 +33,8 @@ constexpr size_t step_cta_smem()
 
 template <class Mdl, int M, int E, int RES>
 __global__ void __launch_bounds__(M / E, pf_min_blocks(M / E, pf_k1_warps(Mdl::S)))
-    k_step_cta(const FilterDesc* __restrict__ descs, StepState X, InputRef in, int32_t* step_ctr)
+    k_step_cta(const FilterDesc* __restrict__ descs, StepState X, const __grid_constant__ InputRef in,
+               int32_t* step_ctr)
 {
     constexpr int NT = M / E, S = Mdl::S, K = Mdl::K, NA = Mdl::NA;
     constexpr int NANG = NA > 0 ? NA : 1;
