@@ -969,23 +969,25 @@ __device__ __forceinline__ int ref_binary_search(const float* hay, float needle,
 
 // Block-wide exclusive count of `flag` in ascending rank order where rank =
 // tid + nt*round; returns this thread's exclusive count, *total the sum.
-// red needs 33 ints.  Contains barriers: every thread must call.
+// red: NT / 32 ints (NT threads); callers alternate between two buffers, so
+// that the one barrier, which every thread must reach, also frees the buffer
+// before.
+template <int NT>
 __device__ __forceinline__ int block_excl_count(bool flag, int* red, int* total)
 {
-    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     const unsigned b = __ballot_sync(kFull, flag);
-    const int in_warp = __popc(b & ((1u << lane) - 1u));
-    __syncthreads();
     if (lane == 0) red[wp] = __popc(b);
     __syncthreads();
     int before = 0, tot = 0;
-    for (int i = 0; i < nw; ++i) {
+#pragma unroll
+    for (int i = 0; i < NT / 32; ++i) {
         const int c = red[i];
         if (i < wp) before += c;
         tot += c;
     }
     *total = tot;
-    return before + in_warp;
+    return before + __popc(b & ((1u << lane) - 1u));
 }
 
 // Vose alias table of M weights (resampling-valias.cl:85-195 + 262-270) in
@@ -993,29 +995,44 @@ __device__ __forceinline__ int block_excl_count(bool flag, int* red, int* total)
 // 1/M), prob = p*M, small iff prob <= 1, pairing prob_L = (prob_L + prob_S) - 1.
 // Work lists are filled in ascending slot order where the reference uses
 // atomic_inc / atomic_dec (the oracle does the same).  Shared: prob[M],
-// alias[M], sl[M], scratch[M] floats, red[33].
+// alias[M], sl[M], scratch[M] floats, red[32].  M / E threads.
+//
+// Bound: barriers and the serial chain of pairing rounds.  A round of more
+// than 32 pairs meets two barriers (one count of the small entries, from which
+// the large ones' ranks follow, and the round's end) and keeps its pairs in
+// registers; it met six and kept them in local memory, sized for one warp.
+// Resampling kernel at 2^20 particles in sub-filters of 512: 27.7 -> 21.0 us.
 template <int M, int E>
 __device__ void vose_build(const float (&w)[E], float* prob, unsigned* alias, unsigned* sl,
                            float* scratch, int* red)
 {
-    const int tid = threadIdx.x, nt = blockDim.x;
+    constexpr int NT = M / E;
+    static_assert(NT <= 512, "two buffers of 16 counts in red");
+    const int tid = threadIdx.x;
 #pragma unroll
     for (int e = 0; e < E; ++e) scratch[E * tid + e] = w[e];
     __syncthreads();
-    // sum_reduce4
+    // sum_reduce4; the levels of at most 32 sums within the first warp
     int offset = M;
     while (offset > 2) {
         offset >>= 2;
-        for (int l = tid; l < offset; l += nt) {
-            const float x = scratch[l + offset] + scratch[l + offset + offset] + scratch[l + offset + offset + offset];
-            scratch[l] = scratch[l] + x;
+        if (offset > 32) {
+            for (int l = tid; l < offset; l += NT) {
+                const float x = scratch[l + offset] + scratch[l + offset + offset] + scratch[l + offset + offset + offset];
+                scratch[l] = scratch[l] + x;
+            }
+            __syncthreads();
+        } else if (tid < 32) {
+            if (tid < offset) {
+                const int l = tid;
+                const float x = scratch[l + offset] + scratch[l + offset + offset] + scratch[l + offset + offset + offset];
+                scratch[l] = scratch[l] + x;
+            }
+            __syncwarp();
         }
-        __syncthreads();
     }
-    if (offset > 1) {
-        if (tid == 0) scratch[0] = scratch[0] + scratch[1];
-        __syncthreads();
-    }
+    if (offset > 1 && tid == 0) scratch[0] = scratch[0] + scratch[1];
+    __syncthreads();
     const float sum = scratch[0];
     // normalise, scale, initial split (small ascending from 0, large descending from M-1)
     int ns_before = 0;
@@ -1035,19 +1052,21 @@ __device__ void vose_build(const float (&w)[E], float* prob, unsigned* alias, un
         fl[e] = prob[E * tid + e] <= 1.0f;
         my_small += fl[e] ? 1 : 0;
     }
+    unsigned small_end;
     {
         // exclusive scan of my_small over threads (ascending tid)
-        const int lane = tid & 31, wp = tid >> 5, nw = nt >> 5;
+        const int lane = tid & 31, wp = tid >> 5;
         int inc = my_small;
+#pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const int o = __shfl_up_sync(kFull, inc, d);
             if (lane >= d) inc += o;
         }
-        __syncthreads();
         if (lane == 31) red[wp] = inc;
         __syncthreads();
         int wbase = 0, tot = 0;
-        for (int i = 0; i < nw; ++i) {
+#pragma unroll
+        for (int i = 0; i < NT / 32; ++i) {
             if (i < wp) wbase += red[i];
             tot += red[i];
         }
@@ -1060,14 +1079,11 @@ __device__ void vose_build(const float (&w)[E], float* prob, unsigned* alias, un
             if (fl[e]) sl[s_i++] = (unsigned)i;
             else sl[M - 1 - (l_i++)] = (unsigned)i;
         }
-        __syncthreads();
-        if (tid == 0) red[32] = tot;
+        small_end = (unsigned)tot;
         __syncthreads();
     }
-    unsigned small_end = (unsigned)red[32];
     unsigned large_rend = small_end - 1u;  // = M-1 - n_large
     unsigned small_begin = 0;
-    __syncthreads();
     // Pairing rounds; each retires >= 1 small entry, so <= M rounds.  Round:
     // the first `nactive` smalls take the `nactive` larges at the bottom of the
     // large list as aliases, the larges' reduced probabilities are appended to
@@ -1075,6 +1091,7 @@ __device__ void vose_build(const float (&w)[E], float* prob, unsigned* alias, un
     // order.  Rounds of at most 32 pairs (the common case once the few large
     // weights are being used up) run in warp 0 alone, without CTA barriers.
     const int lane = tid & 31;
+    int flip = 0;  // which half of red the next count uses
     for (int round = 0; round < M;) {
         const unsigned se = small_end;
         const unsigned a = se - small_begin, b = (unsigned)M - se;
@@ -1176,39 +1193,38 @@ __device__ void vose_build(const float (&w)[E], float* prob, unsigned* alias, un
         }
         ++round;
         large_rend += nactive;
-        constexpr int R = (M / 2 + 31) / 32 + 1;  // upper bound on items per thread
+        constexpr int R = (M / 2 + NT - 1) / NT;  // pairs per thread (nactive <= M / 2)
         unsigned lidx[R];
-        float pS[R], pL[R];
-        int nitems = 0;
-        for (unsigned kk = tid, r = 0; kk < nactive && r < (unsigned)R; kk += nt, ++r) {
-            const unsigned sidx = sl[small_begin + kk];
-            lidx[r] = sl[se + kk];
-            pS[r] = prob[sidx];
-            alias[sidx] = lidx[r];
-            pL[r] = prob[lidx[r]];
-            nitems = (int)r + 1;
-        }
-        __syncthreads();
-        unsigned s_base = 0, l_base = 0;
-        const int rounds = (int)((nactive + nt - 1) / nt);
-        for (int r = 0; r < rounds; ++r) {
-            const unsigned kk = (unsigned)tid + (unsigned)r * nt;
-            const bool act = kk < nactive;
-            float nl = 0.0f;
-            bool small = false;
-            if (act && r < nitems) {
-                nl = (pL[r] + pS[r]) - 1.0f;
-                small = nl <= 1.0f;
+        float nl[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const unsigned kk = (unsigned)(tid + r * NT);
+            if (kk < nactive) {
+                const unsigned sidx = sl[small_begin + kk];
+                lidx[r] = sl[se + kk];
+                alias[sidx] = lidx[r];
+                nl[r] = (prob[lidx[r]] + prob[sidx]) - 1.0f;
             }
+        }
+        // (the first count's barrier orders these reads before the writes below)
+        unsigned s_base = 0, l_base = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (r > 0 && (unsigned)(r * NT) >= nactive) break;
+            const bool act = (unsigned)(tid + r * NT) < nactive;
+            const bool small = act && nl[r] <= 1.0f;
+            // the pairs of this pass are those of its first threads, so the
+            // large ones' ranks and count follow from the small ones'
             int tot_s;
-            const int rank_s = block_excl_count(act && small, red, &tot_s);
-            int tot_l;
-            const int rank_l = block_excl_count(act && !small, red, &tot_l);
+            const int rank_s = block_excl_count<NT>(small, red + 16 * (flip & 1), &tot_s);
+            ++flip;
+            const int rank_l = tid - rank_s;
+            const int tot_l = min((int)nactive - r * NT, NT) - tot_s;
             if (act) {
                 const unsigned dst = small ? small_end + s_base + (unsigned)rank_s
                                            : large_rend - l_base - (unsigned)rank_l;
                 sl[dst] = lidx[r];
-                prob[lidx[r]] = nl;
+                prob[lidx[r]] = nl[r];
             }
             s_base += (unsigned)tot_s;
             l_base += (unsigned)tot_l;
