@@ -768,10 +768,8 @@ static pf_status enqueue_step(pf_filter* f, const FilterDesc* desc, InputRef in,
     CU(mark(nullptr));
     if (c.rng == PF_RNG_REFLAYOUT) {
         const int G = c.mtgp_streams;
-        CU(launch_mtgp_blocks(G, f->mtgp, reinterpret_cast<uint32_t*>(f->rbuf), f->rtotal / G, c.mtgp_mask, 1, 0, st));
-        CU(mark("mtgp32"));
-        CU(launch_boxmuller(f->rbuf, (int64_t)f->mi.K * f->T, st));
-        CU(mark("boxmuller"));
+        CU(launch_mtgp_normals(G, f->mtgp, f->rbuf, f->rtotal / G, (int64_t)f->mi.K * f->T, c.mtgp_mask, st));
+        CU(mark("mtgp32_boxmuller"));
     }
     if (f->pipe == PF_PIPELINE_FUSED) {
         CU(f->ops.step(M, E, c.resampler, N, st, desc, f->X, in, ctr_inc, false));
@@ -812,7 +810,8 @@ static pf_status enqueue_step(pf_filter* f, const FilterDesc* desc, InputRef in,
             CU(f->ops.exchange_inplace(N, nx < 1024 ? ((nx + 31) / 32) * 32 : 1024, st, desc, nullptr));
             CU(mark("exchange"));
         }
-        CU(f->ops.exchange_resample(M, E, c.resampler, N + estimate_ctas(N), st, desc, nullptr, in, ctr_inc, 0));
+        // (every kernel after the generator is a programmatic dependent of the one before it)
+        CU(f->ops.exchange_resample(M, E, c.resampler, N + estimate_ctas(N), st, desc, nullptr, in, ctr_inc, 2));
         CU(mark("resample"));
     }
     if (f->timing) f->nphase = np - 1;

@@ -98,6 +98,60 @@ __global__ void __launch_bounds__(256) k_mtgp_blocks(uint32_t* __restrict__ stat
     mtgp_store(ms, gst, (int)size);
 }
 
+// A filter step's random buffer in one launch: stream g's next `size` words as
+// k_mtgp_blocks, the words whose place in the whole buffer lies below nn (the
+// normals) turned pair by pair into normals by Box-Muller on the way out, the
+// same values as k_mtgp_blocks followed by k_boxmuller.  Each chunk of 2048
+// words is generated in shared memory first, so that the Box-Muller chains of a
+// chunk run side by side instead of inside the barrier-separated rounds.
+//
+// Bound: the recursion's rounds (256 words each, one barrier apart) on as many
+// CTAs as there are streams.  120 streams x 3072 words: 6.8 us; k_mtgp_blocks and
+// k_boxmuller took 7.5 + 3.2 us.
+constexpr int kNormalsThreads = 256, kNormalsChunk = 2048;
+__global__ void __launch_bounds__(kNormalsThreads) k_mtgp_normals(uint32_t* __restrict__ states, float* __restrict__ out,
+                                                                  int64_t size, int64_t nn, uint32_t mask)
+{
+    __shared__ __align__(16) MtgpLinear<kNormalsChunk> ms;
+    __shared__ __align__(16) float raw[kNormalsChunk];
+    allow_dependents();
+    const int g = blockIdx.x, tid = threadIdx.x;
+    uint32_t* gst = states + (int64_t)g * kMtgpN;
+    float* o = out + (int64_t)g * size;
+    mtgp_load_linear<kNormalsThreads>(ms, gst, g % kMtgpSets, mask, [] {});
+    int n = 0;
+    for (int64_t c0 = 0; c0 < size; c0 += kNormalsChunk) {
+        if (c0 > 0) {  // the state to the front
+            constexpr int R = (kMtgpN + kNormalsThreads - 1) / kNormalsThreads;
+            uint32_t w[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) w[r] = ms.x[n + min(tid + r * kNormalsThreads, kMtgpN - 1)];
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (tid + r * kNormalsThreads < kMtgpN) ms.x[tid + r * kNormalsThreads] = w[r];
+            __syncthreads();
+        }
+        n = (int)(size - c0 < kNormalsChunk ? size - c0 : kNormalsChunk);  // even: size is a multiple of 768
+        mtgp_generate_linear<true, kNormalsThreads>(ms, n, n, raw, [] {}, [](int, uint32_t) {});
+        const int64_t left = nn - ((int64_t)g * size + c0);  // normals from here on
+#pragma unroll 4
+        for (int k = 2 * tid; k < n; k += 2 * kNormalsThreads) {
+            float2 v = *reinterpret_cast<const float2*>(raw + k);
+            if (k < left) box_muller(v.x, v.y, v.x, v.y);
+            *reinterpret_cast<float2*>(o + c0 + k) = v;
+        }
+    }
+    mtgp_store_linear(ms, gst, n, 0);
+}
+
+cudaError_t launch_mtgp_normals(int G, uint32_t* states, float* out, int64_t size, int64_t nn, uint32_t mask,
+                                cudaStream_t st)
+{
+    k_mtgp_normals<<<G, kNormalsThreads, 0, st>>>(states, out, size, nn, mask);
+    return cudaGetLastError();
+}
+
 // In-place Box-Muller over pairs (2i, 2i+1) with 2i < n.
 __global__ void k_boxmuller(float* __restrict__ data, int64_t n)
 {

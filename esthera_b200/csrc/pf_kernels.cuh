@@ -515,6 +515,8 @@ __global__ void __launch_bounds__(M / E) k_sample_weight(const FilterDesc* __res
     const int64_t T = D.T;
     const int64_t base = (int64_t)b * M + E * tid;
     if (tid < 32) Mdl::prepare(cst, *input_of(in, f), D.mp, tid);
+    wait_prerequisites();
+    allow_dependents();
     __syncthreads();
     float st[E][S];
 #pragma unroll
@@ -559,6 +561,8 @@ __global__ void __launch_bounds__(M / E) k_block_sort(const FilterDesc* __restri
     const int tid = threadIdx.x;
     const int64_t T = D.T;
     const int64_t base = (int64_t)b * M + E * tid;
+    wait_prerequisites();
+    allow_dependents();
     float* stage = reinterpret_cast<float*>(smem);
     float* sk = stage + (size_t)S * M;
     int* si = reinterpret_cast<int*>(sk + M);
@@ -679,6 +683,8 @@ __global__ void k_exchange_inplace(const FilterDesc* __restrict__ descs, const i
     int f, b;
     cta_target(cta_map, f, b);
     const FilterDesc& D = descs[f];
+    wait_prerequisites();
+    allow_dependents();
     const int nx = exchange_count(D);
     for (int x = threadIdx.x; x < nx; x += blockDim.x) {
         const int64_t d = (int64_t)b * D.M + D.M - 1 - x;

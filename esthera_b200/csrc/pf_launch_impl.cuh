@@ -77,8 +77,7 @@ cudaError_t Launch<Mdl>::sample_weight(int M, int E, int grid, cudaStream_t st, 
 {
 #define PF_SW(m, e)                                                       \
     if (M == m && E == e) {                                               \
-        k_sample_weight<Mdl, m, e><<<grid, m / e, 0, st>>>(d, map, in);   \
-        return cudaGetLastError();                                        \
+        return launch_maybe_dependent(true, k_sample_weight<Mdl, m, e>, grid, m / e, 0, st, d, map, in); \
     }
     PF_ME_LIST(PF_SW)
 #undef PF_SW
@@ -94,8 +93,7 @@ cudaError_t Launch<Mdl>::block_sort(int M, int E, int grid, cudaStream_t st, con
         constexpr size_t sm = (size_t)Mdl::S * m * 4 + (size_t)m * 8;   \
         cudaError_t r = allow_smem(fn, sm);                             \
         if (r != cudaSuccess) return r;                                 \
-        fn<<<grid, m / e, sm, st>>>(d, map);                            \
-        return cudaGetLastError();                                      \
+        return launch_maybe_dependent(true, fn, grid, m / e, sm, st, d, map); \
     }
     PF_ME_LIST(PF_BS)
 #undef PF_BS
@@ -115,8 +113,7 @@ template <class Mdl>
 cudaError_t Launch<Mdl>::exchange_inplace(int grid, int threads, cudaStream_t st, const FilterDesc* d,
                                           const int2* map)
 {
-    k_exchange_inplace<Mdl::S><<<grid, threads, 0, st>>>(d, map);
-    return cudaGetLastError();
+    return launch_maybe_dependent(true, k_exchange_inplace<Mdl::S>, grid, threads, 0, st, d, map);
 }
 
 template <class Mdl>
