@@ -18,8 +18,8 @@ value:  device-timed (CUDA events on the filter's stream), inputs resident
         in HBM, one CUDA-graph replay per step, L2 flushed (256 MB write)
         before every timed step.  value = particles * steps / sum(step time).
 e2e:    the same through the public API with host inputs: pf_step_submit /
-        pf_step_collect (pipelined; H2D of the 128-byte step input and D2H
-        of the estimate for every step inside the timed region, the L2 flush
+        pf_step_collect (pipelined; the 128-byte step input to the device and
+        the estimate back for every step inside the timed region, the L2 flush
         time subtracted); e2e.sync: pf_step, one synchronous step at a time.
 roofline: the dominant kernel's algorithmic bytes (the sampling kernel reads
         the state, 12 B per unicycle particle; the resampling kernel writes
@@ -551,16 +551,16 @@ def main():
         for name, ms in f.last_step_timing():
             phase_ms.setdefault(name, []).append(ms)
     f.set_timing(False)
-    # one untimed submit / collect: it captures the step graph over the pinned
-    # rings (set-up done once per filter, like the device run's warm-up)
+    # one untimed submit / collect: it sets up the pinned ring (once per filter,
+    # like the device run's warm-up)
     f.submit(E.step_input(inputs[0]))
     f.collect()
     f.set_initial_state(np.array(p.init_state[:E.model_info(W["model"])[0]], np.float32))
 
-    # end to end through the public API, pipelined: pf_step_submit (host input
-    # -> pinned ring -> H2D on an upload stream, the step graph waiting for it)
-    # and pf_step_collect (estimate D2H on a download stream into a pinned
-    # ring).  L2 is flushed before every step on the filter's stream; the
+    # end to end through the public API, pipelined: pf_step_submit (the host
+    # input goes to the device as parameters of the step's launches) and
+    # pf_step_collect (the kernels write the estimate into a pinned ring).  L2 is
+    # flushed before every step on the filter's stream; the
     # flushes carry events of their own and their time is subtracted.
     K = args.e2e_steps
     fl = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(K)]

@@ -473,7 +473,7 @@ cudaError_t launch_shard_estimate(const FilterDesc& D, int S, const float* best_
     return cudaErrorInvalidValue;
 }
 
-// A run's device step counter, advanced (or set) by a launch of its own once
+// A run's device step counter, advanced by a launch of its own once
 // every kernel of the step that reads it is enqueued before it.
 __global__ void k_counter_add(int32_t* ctr, int32_t n)
 {

@@ -825,6 +825,16 @@ __device__ __forceinline__ int upper_count(const double* cum, double x)
     return lo < M ? lo : M - 1;
 }
 
+// First i in [0, M] with (u0 + i) * step >= t, from any start.  A call of its
+// own: rarely taken, and inlined at every boundary it would only make the
+// kernel's code, which a launch fetches from memory, longer.
+static __device__ __noinline__ int first_output(double u0, double step, double t, int i, int M)
+{
+    while (i > 0 && (u0 + (double)(i - 1)) * step >= t) --i;
+    while (i < M && (u0 + (double)i) * step < t) ++i;
+    return i;
+}
+
 // Systematic selection from the inclusive sums (scan_f64: this thread's cum[e]
 // and the previous thread's last sum `prev`) by interval boundaries: input j
 // is selected by the outputs i with cum[j-1] <= pos(i) < cum[j],
@@ -850,12 +860,7 @@ __device__ __forceinline__ void systematic_select(const double (&cum)[E], double
     const int tid = threadIdx.x;
     constexpr int W = 32 * E;  // outputs of a warp
     const double u0 = (double)u0f;
-    auto pos = [&](int i) { return (u0 + (double)i) * step; };
-    auto exact = [&](int i, double t) {  // first i in [0, M] with pos(i) >= t, from any start
-        while (i > 0 && pos(i - 1) >= t) --i;
-        while (i < M && pos(i) < t) ++i;
-        return i;
-    };
+    auto exact = [&](int i, double t) { return first_output(u0, step, t, i, M); };
     const int j0 = E * tid;
     int first[E + 1];  // first output at or above the sum before input j0 + e
     // 1 / step by two Newton steps from the FP32 reciprocal of its mantissa: t /
@@ -1531,13 +1536,16 @@ struct DhArm {
         acc = fmaf(d5, d5, acc);
         return -0.5f * acc;
     }
-    // E particles at once (E even): step()'s arithmetic in the same order for
-    // two particles to a packed instruction (F2), bit-identical results.
+    // E particles at once: step()'s arithmetic in the same order, two particles
+    // to a packed instruction (F2, bit-identical results) where E is a multiple
+    // of 4.  With 2 the pair's chain does not fit beside the two states in 72
+    // registers: the sampling kernel at 2^18 particles takes 28.7 us packed and
+    // 25.0 us one by one (L2 flushed; warm 397 and 388 us per 16 steps).
     template <int E, class Noise>
     __device__ static __forceinline__ void step_batch(const Consts& c, float (&s)[E][S], Noise noise,
                                                       float (&sn)[E][NA], float (&cs)[E][NA], float (&ll)[E])
     {
-        if constexpr (E % 2 != 0) {
+        if constexpr (E % 4 != 0) {
 #pragma unroll
             for (int e = 0; e < E; ++e) {
                 float n[K];
@@ -2056,7 +2064,9 @@ __device__ __forceinline__ void model_step_tp(const typename Mdl::Consts& c, flo
 // only by coincidence, so their sub-filters sort with rank_sort_desc.  The
 // DH arm is not one (a resampled duplicate's joint angles advance with the
 // velocity of the previous step, before its noise, so duplicates keep equal
-// keys), nor, conservatively, are the reference's arms.
+// keys).  The camera arms would qualify but gain nothing: with 9 rows to
+// scatter, 16 single-kernel steps of 128 sub-filters of 512 take 127 us so and
+// 125 us with the (key, index) network.
 template <class Mdl>
 struct RareTies : std::false_type {};
 template <>

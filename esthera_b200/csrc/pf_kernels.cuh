@@ -106,11 +106,14 @@ __device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcont
 // Register budgets of the split pipeline's kernels, as resident warps per SM
 // asked of the compiler: __launch_bounds__(threads, ceil(warps * 32 / threads))
 // caps the registers at 65536 / (that many threads).  Small states (the
-// unicycle's 3 variables) take 36 / 32 warps: 16 steps of 2^20 particles (m =
+// unicycle's 3 variables) take 36 warps in the sampling kernel: 16 steps of 2^20 particles (m =
 // 512, 4 particles per thread) take 517 us at 56 or 64 registers of the
 // sampling kernel, 526 us at 72; 6M particles in sub-filters of 256 take 6255
 // us at 56 and 6277 us at 64.  The arms' states (9-12 variables, forward
-// kinematics) need ~128 registers per thread; capping them lower spills.
+// kinematics) take 12 warps (168 registers at 4 particles per thread): 1.1M
+// DH-arm particles in sub-filters of 256, 32 steps, 3107 us against 3375 at 16
+// warps (128 registers, spilling) and 3958 at 20.  The single-kernel step keeps
+// 16 for them.
 // The sampling kernel with two threads per particle asks for 4 warps fewer
 // (its CTAs are twice as large, so the rounding up of whole CTAs would
 // otherwise cut its registers below the one-thread kernel's).
@@ -118,7 +121,7 @@ __device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcont
 #define PF_K1_WARPS_SMALL 36
 #endif
 #ifndef PF_K1_WARPS_LARGE
-#define PF_K1_WARPS_LARGE 16
+#define PF_K1_WARPS_LARGE 12
 #endif
 #ifndef PF_K2_WARPS_SMALL
 #define PF_K2_WARPS_SMALL 32
@@ -131,10 +134,9 @@ __host__ __device__ constexpr int pf_min_blocks(int threads, int warps)
     return (warps * 32 + threads - 1) / threads > 32 ? 32 : (warps * 32 + threads - 1) / threads;
 }
 // Large states with 2 or fewer particles per thread hold half the registers a
-// thread of 4 needs: their budget is 28 warps (72 registers: the packed
-// kinematic chain of the DH arm at m = 256 spills less than at 64, and 2^18
-// particles still fit one wave; 16 steps of 2^18 particles 292 us, against 307
-// at 32 warps and 297 at 24).
+// thread of 4 needs: their budget is 28 warps (72 registers: the DH arm at m =
+// 256 spills less than at 64, and 2^18 particles still fit one wave; sampling
+// kernel 25.0 us with the L2 flushed, against 26.7 at 32 warps).
 #ifndef PF_K1_WARPS_LARGE_E2
 #define PF_K1_WARPS_LARGE_E2 28
 #endif
@@ -142,6 +144,10 @@ __host__ __device__ constexpr int pf_k1_warps(int S, int E = 4)
 {
     return S <= 3 ? PF_K1_WARPS_SMALL : (E <= 2 ? PF_K1_WARPS_LARGE_E2 : PF_K1_WARPS_LARGE);
 }
+__host__ __device__ constexpr int pf_step_warps(int S) { return S <= 3 ? PF_K1_WARPS_SMALL : 16; }
+// The resampling kernel of a small state keeps 32 warps (64 registers): 40 (48)
+// runs 6M particles in sub-filters of 256 2.4 % faster but a filter of 256 such
+// sub-filters, whose step is one CTA's latency, 6 % slower.
 __host__ __device__ constexpr int pf_k2_warps(int S) { return S <= 3 ? PF_K2_WARPS_SMALL : PF_K2_WARPS_LARGE; }
 
 struct InputRef {
@@ -828,12 +834,10 @@ __device__ __forceinline__ double weighted_rows_staged(const double* rows, int r
 // aligned): every row arrives in one round of copies before the maximum and
 // the sums; otherwise the maximum's values load first and the rows after.
 // The same result either way.
-// Returns lane j's sum j; gl, wk, wi: the maximum and the winner (sub-filter
-// idx0 + wi).
 template <int S, bool STAGED = false>
-__device__ __forceinline__ double group_sums(const FilterDesc& D, const double* __restrict__ part,
-                                             const float* __restrict__ winner, int nr, int NV, int lane, double& gl,
-                                             float& wk, int& wi, double* stage = nullptr)
+__device__ __forceinline__ void group_row(const FilterDesc& D, const double* __restrict__ part,
+                                          const float* __restrict__ winner, int nr, int NV, int idx0, int lane,
+                                          double* __restrict__ go, double* stage = nullptr)
 {
     const bool valid = lane < nr;
     if constexpr (STAGED) stage_rows(stage, part, nr, NV, lane);
@@ -846,9 +850,9 @@ __device__ __forceinline__ double group_sums(const FilterDesc& D, const double* 
     } else {
         l = valid ? __ldcg(part + (int64_t)lane * kPartStride) : -INFINITY;
     }
-    gl = l;
-    wk = lw;
-    wi = valid ? lane : 0x7fffffff;
+    double gl = l;
+    float wk = lw;
+    int wi = valid ? lane : 0x7fffffff;
     auto reduce = [&] {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -862,25 +866,14 @@ __device__ __forceinline__ double group_sums(const FilterDesc& D, const double* 
         }
         return valid ? (D.log_weights ? exp(l - gl) : 1.0) : 0.0;
     };
+    double a;
     if constexpr (STAGED) {
-        return weighted_rows_staged(stage, staged_stride(NV), nr, reduce(), NV, lane);
+        a = weighted_rows_staged(stage, staged_stride(NV), nr, reduce(), NV, lane);
     } else if constexpr (2 + 2 * S <= 8) {
-        return weighted_rows(part, nr, reduce(), NV, lane);
+        a = weighted_rows(part, nr, reduce(), NV, lane);
     } else {
-        return weighted_rows_late(part, nr, NV, lane, reduce);
+        a = weighted_rows_late(part, nr, NV, lane, reduce);
     }
-}
-
-// The row itself, into go.
-template <int S, bool STAGED = false>
-__device__ __forceinline__ void group_row(const FilterDesc& D, const double* __restrict__ part,
-                                          const float* __restrict__ winner, int nr, int NV, int idx0, int lane,
-                                          double* __restrict__ go, double* stage = nullptr)
-{
-    double gl;
-    float wk;
-    int wi;
-    const double a = group_sums<S, STAGED>(D, part, winner, nr, NV, lane, gl, wk, wi, stage);
     if (lane >= 1 && lane < NV) go[lane] = a;
     if (lane == 0) {
         go[0] = D.log_weights ? gl : 0.0;
@@ -1069,39 +1062,20 @@ __device__ __forceinline__ void estimate_group(const FilterDesc& D, int g, const
     const int b = g << 5, ng = (D.N + 31) >> 5;
     const int NV = 2 + S + D.na;
     const int32_t step_no = in.ctr ? *in.ctr + in.add + 1 : 0;
-    if (ng == 1 && !D.shard) {
-        // one group: its sums are the filter's (the second level would scale
-        // them by exp(0)), without the ticket and the row's way through memory
-        // (8 sub-filters stepped from the host: 306 -> 297 us per 8 steps)
-        double gl;
-        float wk;
-        int wi;
-        const double a = group_sums<S, STAGED>(D, D.part, D.winner, D.N, NV, lane, gl, wk, wi, smem);
-        wk = __shfl_sync(kFull, wk, 0);
-        wi = __shfl_sync(kFull, wi, 0);
-        const bool won = wk >= -INFINITY;  // a NaN key never wins
-        const int best = won && wi < D.N ? wi : 0;
-        const int bv = lane - PF_MAX_STATE;
-        const float best_v = (bv >= 0 && bv < S) ? __ldcg(D.tmp + bv * D.T + (int64_t)best * D.M) : 0.0f;
-        estimate_store<S>(D, lane, NV, D.log_weights ? gl : 0.0, won ? wk : -INFINITY, best, best_v, 0.0 + a,
-                          D.est[step_index(in)], step_no);
-        if (lane == 0) {
-            publish_estimate(in);
-            if (step_ctr) *step_ctr += in.inc;
-        }
-        return;
-    }
     // winners as filter-wide indices (a shard's sub-filters start at b0)
     group_row<S, STAGED>(D, D.part + (int64_t)b * kPartStride, D.winner + b, min(32, D.N - b), NV, b + D.b0, lane,
                          D.gpart + (int64_t)g * kPartStride, smem);
     if (D.shard) return;  // the shards' group rows are combined across shards (pf_shard_estimate)
     __syncwarp();
     __threadfence();
-    int last = 0;
-    if (lane == 0) last = atomicAdd(D.est_ctr, 1) == ng - 1;
-    last = __shfl_sync(kFull, last, 0);
-    if (!last) return;
-    __threadfence();
+    if (ng > 1) {  // (a single group is the last one: no ticket)
+        int last = 0;
+        if (lane == 0) last = atomicAdd(D.est_ctr, 1) == ng - 1;
+        last = __shfl_sync(kFull, last, 0);
+        if (!last) return;
+        __threadfence();
+    }
+    __syncwarp();
     if constexpr (STAGED) {
         const int wr = (CAP / staged_stride(NV + 2)) & ~31;
         estimate_final_staged<S>(D, lane, ng, NV, D.tmp, D.est[step_index(in)], step_no, smem, wr);
@@ -1109,7 +1083,7 @@ __device__ __forceinline__ void estimate_group(const FilterDesc& D, int g, const
         estimate_final<S>(D, lane, ng, NV, D.tmp, D.est[step_index(in)], step_no);
     }
     if (lane == 0) {
-        *D.est_ctr = 0;
+        if (ng > 1) *D.est_ctr = 0;
         publish_estimate(in);
         __threadfence();
         if (step_ctr) *step_ctr += in.inc;

@@ -242,13 +242,14 @@ pf_status pf_get_sorted(pf_filter* f, float* soa, float* keys);
 pf_status pf_get_selection(pf_filter* f, int32_t* sel);
 /* Turn recording of the resampling selections on or off (off by default: it costs 4 bytes per particle-step). */
 pf_status pf_record_selection(pf_filter* f, int32_t enable);
-/* One step with host inputs (copied H2D) and a host estimate (copied D2H); synchronous. */
+/* One step with a host input (carried by the launches) and a host estimate (written to pinned memory); synchronous. */
 pf_status pf_step(pf_filter* f, const pf_step_input* in, pf_estimate* out);
 /* Device-resident run: d_inputs[capacity] and d_estimates[capacity] in device
  * memory; resets the step counter and runs `steps` steps (step k reads
  * d_inputs[k % capacity], writes d_estimates[k % capacity]).  Asynchronous on
- * the filter's stream: one step is captured into a CUDA graph (once per
- * argument set) and replayed with a device step counter.  pf_synchronize() waits. */
+ * the filter's stream: one step -- and, once the filter has run 64, four and
+ * sixteen steps -- is captured into a CUDA graph (once per argument set) and
+ * replayed with a device step counter.  pf_synchronize() waits. */
 pf_status pf_run_device(pf_filter* f, const pf_step_input* d_inputs, pf_estimate* d_estimates,
                         int32_t capacity, int32_t steps);
 /* Replays `steps` more steps of the run set up by pf_run_device (the step
@@ -256,19 +257,17 @@ pf_status pf_run_device(pf_filter* f, const pf_step_input* d_inputs, pf_estimate
 pf_status pf_run_device_continue(pf_filter* f, int32_t steps);
 /* Pipelined host stepping (no counterpart in the reference, whose driver loop
  * copies each step's estimate back before the next step starts,
- * pf_generic_soa.cu:858-1154).  pf_step_submit copies the input into a pinned
- * ring slot and returns without waiting: the slot is uploaded on a copy stream,
- * the step (the CUDA graph of pf_run_device, over device rings of
- * PF_QUEUE_DEPTH inputs and estimates) runs on the filter's stream once the
- * upload landed, and the estimate is downloaded into a pinned ring slot on a
- * second copy stream, so uploads and downloads overlap the neighbouring steps.
- * Results equal pf_step's on the same inputs (the step counter is the number of
- * steps since the initial state, as for pf_step).  At most PF_QUEUE_DEPTH steps
- * may be pending: a further submit returns PF_ERR_BUSY, as does a submit after
- * another call stepped the filter while steps are pending.
+ * pf_generic_soa.cu:858-1154).  pf_step_submit enqueues one step and returns
+ * without waiting: the input travels with the step's launches, which follow the
+ * step before's (programmatic dependent launch, so a step's random numbers are
+ * generated while the step before ends), and the kernels write the estimate into a
+ * pinned ring of PF_QUEUE_DEPTH slots.  Results equal pf_step's on the same inputs
+ * (the step number counts from the initial state, as for pf_step).  At most
+ * PF_QUEUE_DEPTH steps may be pending: a further submit returns PF_ERR_BUSY, as
+ * does a submit after another call stepped the filter while steps are pending.
  * pf_step_collect returns up to `max` estimates in submission order; wait != 0
- * blocks until that many are done (or all pending ones), wait == 0 returns the
- * finished ones only.  One host thread per filter. */
+ * blocks until that many are there (or all pending ones), wait == 0 returns those
+ * that are.  One host thread per filter. */
 #define PF_QUEUE_DEPTH 64
 pf_status pf_step_submit(pf_filter* f, const pf_step_input* in);
 pf_status pf_step_collect(pf_filter* f, pf_estimate* out, int32_t max, int32_t wait, int32_t* count);
@@ -559,8 +558,8 @@ pf_status pfk_estimate(const float* keys, const float* state, int32_t num_state,
  * owns every allocation, the allocator is locked after start-up, or no
  * allocation may happen between stream captures).  No counterpart in the
  * reference.  Inputs and output are device pointers the caller owns; it calls
- * no cudaMalloc/cudaFree: its per-sub-filter scratch is a static device array
- * sized for at most 4096 sub-filters (num_particles / m), about 1.15 MB held
+ * no cudaMalloc/cudaFree: its scratch is a static device array
+ * sized for at most 4096 sub-filters (num_particles / m), about 1.18 MB held
  * by every GPU that loads the library.  Larger inputs return PF_ERR_INVALID.
  * The first call on a device looks up the array's device address (make that
  * call before any stream capture); the address is kept per device and CUDA

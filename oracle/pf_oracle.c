@@ -597,7 +597,7 @@ static int is_angle(const orc_model* md, int v)
 /* exp(x) for max-subtracted log-weights x <= 0 from correctly rounded FP32
  * operations only: n = rint(x log2 e), r = x - n ln2 (Cody-Waite, two fmaf),
  * exp(x) = 2^n P(r) with the project's degree-6 fit of P (the engine's
- * pf_expneg evaluates the same operations in the same order, so both give the
+ * pf_expneg2 evaluates the same operations in the same order, so both give the
  * same bits; esthera_b200/csrc/fit_exp.py fits and checks the polynomial).
  * x < -87 (and -inf) gives 0; NaN stays NaN. */
 float orc_expneg(float x)
