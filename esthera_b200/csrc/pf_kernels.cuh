@@ -1,19 +1,18 @@
 // pf_kernels.cuh -- kernels of the particle-filter step (sm_100a).
 //
 // Split pipeline (two launches per step; batches and the server use it too):
-//   k_sample_sort       one CTA per sub-filter: MTGP32 stream -> Box-Muller in
-//                       shared memory -> propagate + log-weight (float4 SoA
-//                       loads) -> bitonic sort -> sorted state/keys, winner,
-//                       FP64 estimate partials
+//   k_sample_sort       one CTA per sub-filter: MTGP32 stream -> Box-Muller ->
+//                       propagate + log-weight (float4 SoA loads) -> FP64
+//                       estimate partials -> sort -> sorted state/keys, winner
 //   k_a2a_merge         (all-to-all exchange only) global top-t of the sorted lists
-//   k_exchange_resample one CTA per sub-filter, estimate-combining group
-//                       leaders first: neighbours' top-t into the weakest
-//                       slots, weights, resampling, gather, store
+//   k_exchange_resample one estimate CTA per 32 sub-filters, then one CTA per
+//                       sub-filter: neighbours' top-t into the weakest slots,
+//                       weights, resampling, gather, store
 // Single-kernel pipeline: k_step_cta (pf_step_cta.cuh), the same phases in one
 // launch with the resampling deferred to the next step.
 // Phased pipeline (the reference's kernel sequence, pf_generic_soa.cu:842-1234):
-//   k_mtgp_blocks -> k_boxmuller -> k_sample_weight -> k_block_sort ->
-//   k_exchange_inplace -> k_exchange_resample (estimate combined at its start)
+//   k_mtgp_normals -> k_sample_weight -> k_block_sort -> k_exchange_inplace ->
+//   k_exchange_resample (estimate combined at its start)
 #pragma once
 
 #include "pf_device.cuh"
