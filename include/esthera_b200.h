@@ -565,8 +565,8 @@ pf_status pfk_estimate(const float* keys, const float* state, int32_t num_state,
  * call before any stream capture); the address is kept per device and CUDA
  * context, so the first call after cudaDeviceReset (or from another context
  * on the same device) looks it up again.  All calls share the array and every call
- * overwrites the entries it reads, so nothing needs clearing; calls that
- * overlap on the GPU (other streams, other threads) race on it.
+ * clears or overwrites what it reads there; calls that overlap on the GPU
+ * (other streams, other threads) race on it, and only their own results suffer.
  * Asynchronous on `stream` (a cudaStream_t, NULL = default stream). */
 pf_status pfk_estimate_noalloc(const float* d_keys, const float* d_state, int32_t num_state,
                                int64_t num_particles, int32_t m, uint32_t angle_mask,
