@@ -978,6 +978,11 @@ extern "C" pf_status pf_step_submit(pf_filter* f, const pf_step_input* in)
     CU(cudaSetDevice(f->cfg.device));
     pf_status s = queue_setup(f);
     if (s != PF_OK) return s;
+    // captured launches would not run, and the step would stay pending for good
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CU(cudaStreamIsCapturing(f->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone)
+        return fail(PF_ERR_CUDA, "a submitted step cannot be captured (the filter's stream is capturing)");
     if (f->q_pending >= PF_QUEUE_DEPTH)
         return fail(PF_ERR_BUSY, "%d steps pending: collect before submitting more", PF_QUEUE_DEPTH);
     bool chained = f->pipe == PF_PIPELINE_SPLIT && !f->timing;

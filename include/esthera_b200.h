@@ -265,6 +265,7 @@ pf_status pf_run_device_continue(pf_filter* f, int32_t steps);
  * (the step number counts from the initial state, as for pf_step).  At most
  * PF_QUEUE_DEPTH steps may be pending: a further submit returns PF_ERR_BUSY, as
  * does a submit after another call stepped the filter while steps are pending.
+ * A submit while the filter's stream is being captured is refused (PF_ERR_CUDA).
  * pf_step_collect returns up to `max` estimates in submission order; wait != 0
  * blocks until that many are there (or all pending ones), wait == 0 returns those
  * that are.  One host thread per filter. */
