@@ -424,19 +424,14 @@ __device__ __forceinline__ F2 pf_sqrt2(F2 d2)
     d2.get(a, b);
     return d2 * F2(rsqrt_normal(fmaxf(a, 1e-30f)), rsqrt_normal(fmaxf(b, 1e-30f)));
 }
-// (NORMAL: infinite or NaN where the larger coordinate is zero, subnormal or NaN.)
-template <bool NORMAL = false>
+// (pf_atan2_2: infinite or NaN where the larger coordinate is zero, subnormal or NaN.)
 __device__ __forceinline__ F2 pf_atan2_2(F2 y, F2 x)
 {
     float y0, y1, x0, x1;
     y.get(y0, y1);
     x.get(x0, x1);
     const float ax0 = fabsf(x0), ay0 = fabsf(y0), ax1 = fabsf(x1), ay1 = fabsf(y1);
-    auto ratio = [](float u, float v) {
-        const float mn = fminf(u, v), mx = fmaxf(u, v);
-        return NORMAL ? pf_ratio_normal(mn, mx) : pf_ratio(mn, mx);
-    };
-    const F2 a(ratio(ax0, ay0), ratio(ax1, ay1));
+    const F2 a(pf_ratio_normal(fminf(ax0, ay0), fmaxf(ax0, ay0)), pf_ratio_normal(fminf(ax1, ay1), fmaxf(ax1, ay1)));
     const F2 s = a * a;
     F2 p(-4.054567008e-03f);
     p = fma2(p, s, F2(2.186295757e-02f));
@@ -1468,7 +1463,7 @@ struct Unicycle {
                     const F2 er = sub2(rm, r) * isr;
                     const F2 cp = fma2(c2[q], cb, s2[q] * nsb);
                     const F2 sp = fma2(s2[q], cb, c2[q] * sb);
-                    const F2 eb = pf_atan2_2<true>(fma2(sp, dx, cp * ndy), fma2(cp, dx, sp * dy)) * isb;
+                    const F2 eb = pf_atan2_2(fma2(sp, dx, cp * ndy), fma2(cp, dx, sp * dy)) * isb;
                     acc[q] = fma2(er, er, acc[q]);
                     acc[q] = fma2(eb, eb, acc[q]);
                 }
@@ -1491,9 +1486,8 @@ struct DhArm {
     static constexpr int S = 12, K = 6, NA = 6, C = 0, Z = 6;
     __host__ __device__ static constexpr int angle_var(int a) { return a; }
     struct Consts {
-        // each value twice (a packed operand), two to a 16-byte load
         struct alignas(16) Joint {
-            float2 a, d, ca, sa, nca, nsa;
+            float a, d, ca, sa;
         } j[6];
         float dt, sqd, isp, isa;
         float z[6];
@@ -1511,8 +1505,7 @@ struct DhArm {
             const int i = lane;
             float sa, ca;
             sincosf(p.alpha[i], &sa, &ca);
-            c.j[i] = {make_float2(p.a[i], p.a[i]), make_float2(p.d[i], p.d[i]), make_float2(ca, ca),
-                      make_float2(sa, sa), make_float2(-ca, -ca), make_float2(-sa, -sa)};
+            c.j[i] = {p.a[i], p.d[i], ca, sa};
             c.z[i] = in.meas[i];
         }
     }
@@ -1531,10 +1524,10 @@ struct DhArm {
             sn[i] = sq;
             cs[i] = cq;
             // A_i = [[c, -s ca, s sa, a c], [s, c ca, -c sa, a s], [0, sa, ca, d]]
-            const float a00 = cq, a01 = -(sq * c.j[i].ca.x), a02 = sq * c.j[i].sa.x;
-            const float a10 = sq, a11 = cq * c.j[i].ca.x, a12 = -(cq * c.j[i].sa.x);
-            const float a21 = c.j[i].sa.x, a22 = c.j[i].ca.x;
-            const float t0 = c.j[i].a.x * cq, t1 = c.j[i].a.x * sq, t2 = c.j[i].d.x;
+            const float a00 = cq, a01 = -(sq * c.j[i].ca), a02 = sq * c.j[i].sa;
+            const float a10 = sq, a11 = cq * c.j[i].ca, a12 = -(cq * c.j[i].sa);
+            const float a21 = c.j[i].sa, a22 = c.j[i].ca;
+            const float t0 = c.j[i].a * cq, t1 = c.j[i].a * sq, t2 = c.j[i].d;
             const float n00 = fmaf(R01, a10, R00 * a00), n01 = fmaf(R02, a21, fmaf(R01, a11, R00 * a01)),
                         n02 = fmaf(R02, a22, fmaf(R01, a12, R00 * a02));
             const float n10 = fmaf(R11, a10, R10 * a00), n11 = fmaf(R12, a21, fmaf(R11, a11, R10 * a01)),
@@ -1564,75 +1557,6 @@ struct DhArm {
         acc = fmaf(d5, d5, acc);
         return -0.5f * acc;
     }
-    // E particles at once: step()'s arithmetic in the same order, two particles
-    // to a packed instruction (F2, bit-identical results) where E is a multiple
-    // of 4.  With 2 the pair's chain does not fit beside the two states in 72
-    // registers: the sampling kernel at 2^18 particles takes 28.7 us packed and
-    // 25.0 us one by one (L2 flushed; warm 397 and 388 us per 16 steps).
-    template <int E, class Noise>
-    __device__ static __forceinline__ void step_batch(const Consts& c, float (&s)[E][S], Noise noise,
-                                                      float (&sn)[E][NA], float (&cs)[E][NA], float (&ll)[E])
-    {
-        if constexpr (E % 4 != 0) {
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                float n[K];
-#pragma unroll
-                for (int v = 0; v < K; ++v) n[v] = noise(e, v);
-                ll[e] = step(c, s[e], n, sn[e], cs[e]);
-            }
-        } else {
-#pragma unroll
-            for (int e = 0; e < E; e += 2) {
-                F2 R[9], p[3];
-#pragma unroll
-                for (int i = 0; i < 9; ++i) R[i] = F2(i % 4 == 0 ? 1.0f : 0.0f);
-#pragma unroll
-                for (int i = 0; i < 3; ++i) p[i] = F2(0.0f);
-#pragma unroll
-                for (int i = 0; i < 6; ++i) {
-                    const F2 v(s[e][6 + i], s[e + 1][6 + i]);
-                    const F2 q = wrap_pi2(fma2(v, F2(c.dt), F2(s[e][i], s[e + 1][i])));
-                    q.get(s[e][i], s[e + 1][i]);
-                    fma2(F2(c.sqd), F2(noise(e, i), noise(e + 1, i)), v).get(s[e][6 + i], s[e + 1][6 + i]);
-                    F2 sq, cq;
-                    sincos2(q, sq, cq);
-                    sq.get(sn[e][i], sn[e + 1][i]);
-                    cq.get(cs[e][i], cs[e + 1][i]);
-                    const typename Consts::Joint j = c.j[i];
-                    const F2 a01 = sq * F2(j.nca), a02 = sq * F2(j.sa);
-                    const F2 a11 = cq * F2(j.ca), a12 = cq * F2(j.nsa);
-                    const F2 t0 = F2(j.a) * cq, t1 = F2(j.a) * sq;
-#pragma unroll
-                    for (int r = 0; r < 3; ++r) {
-                        const F2 r0 = R[3 * r], r1 = R[3 * r + 1], r2 = R[3 * r + 2];
-                        p[r] = fma2(r2, F2(j.d), fma2(r1, t1, fma2(r0, t0, p[r])));
-                        R[3 * r] = fma2(r1, sq, r0 * cq);
-                        R[3 * r + 1] = fma2(r2, F2(j.sa), fma2(r1, a11, r0 * a01));
-                        R[3 * r + 2] = fma2(r2, F2(j.ca), fma2(r1, a12, r0 * a02));
-                    }
-                }
-                const F2 yaw = pf_atan2_2(R[3], R[0]);
-                const F2 pitch = pf_atan2_2(R[6] * F2(-1.0f), pf_sqrt2(fma2(R[7], R[7], R[8] * R[8])));
-                const F2 roll = pf_atan2_2(R[7], R[8]);
-                F2 acc(0.0f);
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    const F2 d = sub2(F2(c.z[i]), p[i]) * F2(c.isp);
-                    acc = i == 0 ? d * d : fma2(d, d, acc);
-                }
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    F2 d = sub2(F2(c.z[3 + i]), i == 0 ? yaw : (i == 1 ? pitch : roll));
-                    float k0, k1;
-                    (d * F2(kInvTwoPi)).get(k0, k1);
-                    d = fma2(F2(-kTwoPi), F2(rintf(k0), rintf(k1)), d) * F2(c.isa);
-                    acc = fma2(d, d, acc);
-                }
-                (F2(-0.5f) * acc).get(ll[e], ll[e + 1]);
-            }
-        }
-    }
     // Two threads per particle (lane pair h = 0, 1): both lanes advance all
     // joints (identical arithmetic); lane h chains the transforms of joints
     // 3h .. 3h+2 from the identity, the pair swaps chains and joint sines, and
@@ -1659,11 +1583,11 @@ struct DhArm {
             __sincosf(qi, &sq, &cq);
             msn[k] = sq;
             mcs[k] = cq;
-            const float ca = c.j[i].ca.x, sa = c.j[i].sa.x;
+            const float ca = c.j[i].ca, sa = c.j[i].sa;
             const float a00 = cq, a01 = -(sq * ca), a02 = sq * sa;
             const float a10 = sq, a11 = cq * ca, a12 = -(cq * sa);
             const float a21 = sa, a22 = ca;
-            const float t0 = c.j[i].a.x * cq, t1 = c.j[i].a.x * sq, t2 = c.j[i].d.x;
+            const float t0 = c.j[i].a * cq, t1 = c.j[i].a * sq, t2 = c.j[i].d;
             float N[9];
 #pragma unroll
             for (int r = 0; r < 3; ++r) {

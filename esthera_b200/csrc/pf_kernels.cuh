@@ -109,10 +109,12 @@ __device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcont
 // 512, 4 particles per thread) take 517 us at 56 or 64 registers of the
 // sampling kernel, 526 us at 72; 6M particles in sub-filters of 256 take 6255
 // us at 56 and 6277 us at 64.  The arms' states (9-12 variables, forward
-// kinematics) take 12 warps (168 registers at 4 particles per thread): 1.1M
-// DH-arm particles in sub-filters of 256, 32 steps, 3107 us against 3375 at 16
-// warps (128 registers, spilling) and 3958 at 20.  The single-kernel step keeps
-// 16 for them.
+// kinematics) take 16 warps (128 registers at 4 particles per thread).  Against
+// 12 warps (168 registers), 16 steps of sub-filters of 256: camera arm 328
+// against 405 us at 1024 sub-filters and 1078 against 1178 at 4096, the
+// reference's arm 323 against 391 and 1030 against 1140, DH arm 416 against 535
+// and 1442 against 1518; below one wave of the 12 (888 sub-filters) they are
+// equal at 64 and 256, and 12 is ahead by up to 9 % at 768.
 // The sampling kernel with two threads per particle asks for 4 warps fewer
 // (its CTAs are twice as large, so the rounding up of whole CTAs would
 // otherwise cut its registers below the one-thread kernel's).
@@ -120,7 +122,7 @@ __device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcont
 #define PF_K1_WARPS_SMALL 36
 #endif
 #ifndef PF_K1_WARPS_LARGE
-#define PF_K1_WARPS_LARGE 12
+#define PF_K1_WARPS_LARGE 16
 #endif
 #ifndef PF_K2_WARPS_SMALL
 #define PF_K2_WARPS_SMALL 32
@@ -135,7 +137,9 @@ __host__ __device__ constexpr int pf_min_blocks(int threads, int warps)
 // Large states with 2 or fewer particles per thread hold half the registers a
 // thread of 4 needs: their budget is 28 warps (72 registers: the DH arm at m =
 // 256 spills less than at 64, and 2^18 particles still fit one wave; sampling
-// kernel 25.0 us with the L2 flushed, against 26.7 at 32 warps).
+// kernel 25.0 us with the L2 flushed, against 26.7 at 32 warps; 16 steps of 1024
+// sub-filters of 256, 28 against 32 warps: DH arm 386 and 416 us, camera arm 341
+// and 361, the reference's arm 322 and 337).
 #ifndef PF_K1_WARPS_LARGE_E2
 #define PF_K1_WARPS_LARGE_E2 28
 #endif
@@ -143,7 +147,6 @@ __host__ __device__ constexpr int pf_k1_warps(int S, int E = 4)
 {
     return S <= 3 ? PF_K1_WARPS_SMALL : (E <= 2 ? PF_K1_WARPS_LARGE_E2 : PF_K1_WARPS_LARGE);
 }
-__host__ __device__ constexpr int pf_step_warps(int S) { return S <= 3 ? PF_K1_WARPS_SMALL : 16; }
 // The resampling kernel of a small state keeps 32 warps (64 registers): 40 (48)
 // runs 6M particles in sub-filters of 256 2.4 % faster but a filter of 256 such
 // sub-filters, whose step is one CTA's latency, 6 % slower.

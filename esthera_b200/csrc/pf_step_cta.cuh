@@ -32,7 +32,7 @@ constexpr size_t step_cta_smem()
 }
 
 template <class Mdl, int M, int E, int RES>
-__global__ void __launch_bounds__(M / E, pf_min_blocks(M / E, pf_step_warps(Mdl::S)))
+__global__ void __launch_bounds__(M / E, pf_min_blocks(M / E, pf_k1_warps(Mdl::S)))
     k_step_cta(const FilterDesc* __restrict__ descs, StepState X, const __grid_constant__ InputRef in,
                int32_t* step_ctr)
 {
