@@ -142,7 +142,7 @@ bool pfhost::dependent_launch_pays(int grid, int M, int E, int S, int device)
         sms[device].store(n, std::memory_order_relaxed);
     }
     const int wave = n * pf_min_blocks(M / E, pf_k1_warps(S, E));
-    return S <= 3 || 2 * grid <= wave || grid > wave;
+    return S <= 3 || grid > wave || (E <= 2 && 2 * grid <= wave);
 }
 
 extern "C" pf_status pf_model_info(pf_model_id model, int32_t* S, int32_t* K, int32_t* C, int32_t* Z)
@@ -790,8 +790,13 @@ static pf_status enqueue_step(pf_filter* f, const FilterDesc* desc, InputRef in,
         // step counter, so it advances in a launch of its own after the kernel
         const bool late = ctr_inc && c.exchange_period > 1;
         // a programmatic dependent of the sampling kernel when that pays (its
-        // CTAs start during the sampling kernel's last wave and wait there)
-        const int virt = dependent_launch_pays(N, M, E, f->mi.S, c.device) ? 3 : 1;
+        // CTAs start during the sampling kernel's last wave and wait there); of
+        // a step launched from the host always: it hides the second launch
+        // (1024 sub-filters of 256, 16 submitted steps without -> with: DH arm
+        // 38.3 -> 36.1 us a step with other work between the steps, camera arm
+        // 34.3 -> 32.2 so and 383 -> 359 us back to back; 16 synchronous steps
+        // 770 -> 719 and 732 -> 690 us)
+        const int virt = in.inlined || dependent_launch_pays(N, M, E, f->mi.S, c.device) ? 3 : 1;
         CU(f->ops.exchange_resample(M, E, c.resampler, N + estimate_ctas(N), st, desc, nullptr, in,
                                     late ? nullptr : ctr_inc, virt));
         CU(mark("exchange_resample"));

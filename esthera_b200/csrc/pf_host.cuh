@@ -44,7 +44,10 @@ bool model_info(int model, ModelInfo* mi);
 // takes more than half of one wave but not more than one, where the waiting
 // CTAs crowd out the sampling kernel's (DH arm, sub-filters of 256: 20.5 ->
 // 13.6 at 256, 22.1 -> 21.8 at 512, but 23.0 -> 23.4 at 768 and 24.2 -> 25.4 at
-// 1024; 43.8 -> 43.9 at 2048).
+// 1024; 43.8 -> 43.9 at 2048), and with four or more particles per thread not
+// up to one wave either (16 steps without -> with: DH arm 267 -> 302 us at 256
+// and 302 -> 350 at 512, camera arm 205 -> 226 and 249 -> 266; 64 sub-filters
+// 232 -> 231 and 189 -> 180).
 bool dependent_launch_pays(int grid, int M, int E, int S, int device);
 const float* init_state_of(int model, const ModelParams& mp);
 uint32_t angle_mask_of(int model);
