@@ -768,8 +768,15 @@ static pf_status enqueue_step(pf_filter* f, const FilterDesc* desc, InputRef in,
     CU(mark(nullptr));
     if (c.rng == PF_RNG_REFLAYOUT) {
         const int G = c.mtgp_streams;
-        CU(launch_mtgp_normals(G, f->mtgp, f->rbuf, f->rtotal / G, (int64_t)f->mi.K * f->T, c.mtgp_mask, st));
-        CU(mark("mtgp32_boxmuller"));
+        if (f->timing) {  // the reference's two phases apart (the same numbers)
+            CU(launch_mtgp_blocks(G, f->mtgp, reinterpret_cast<uint32_t*>(f->rbuf), f->rtotal / G, c.mtgp_mask, 1, 0,
+                                  st));
+            CU(mark("mtgp32"));
+            CU(launch_boxmuller(f->rbuf, (int64_t)f->mi.K * f->T, st));
+            CU(mark("boxmuller"));
+        } else {
+            CU(launch_mtgp_normals(G, f->mtgp, f->rbuf, f->rtotal / G, (int64_t)f->mi.K * f->T, c.mtgp_mask, st));
+        }
     }
     if (f->pipe == PF_PIPELINE_FUSED) {
         CU(f->ops.step(M, E, c.resampler, N, st, desc, f->X, in, ctr_inc, false));
