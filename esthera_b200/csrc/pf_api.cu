@@ -4,6 +4,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <sched.h>
 #include <mutex>
 #include <string>
 #include <unordered_set>
@@ -1029,6 +1030,12 @@ extern "C" pf_status pf_step_collect(pf_filter* f, pf_estimate* out, int32_t max
     *count = 0;
     if (f->q_pending == 0 || max <= 0) return PF_OK;
     CU(cudaSetDevice(f->cfg.device));
+    // waits poll pinned memory; a device set to yield or to block has the
+    // waiting thread give its core away between polls
+    unsigned flags = 0;
+    if (wait) CU(cudaGetDeviceFlags(&flags));
+    const bool yield = (flags & cudaDeviceScheduleMask) == cudaDeviceScheduleYield ||
+                       (flags & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync;
     while (*count < max && f->q_pending > 0) {
         const int32_t k = f->q_next - f->q_pending;  // oldest pending step
         const int slot = (int)((uint32_t)k % PF_QUEUE_DEPTH);
@@ -1043,6 +1050,7 @@ extern "C" pf_status pf_step_collect(pf_filter* f, pf_estimate* out, int32_t max
                 if (!got && e != cudaErrorNotReady) CU(e);
                 if (e == cudaErrorNotReady) cudaGetLastError();
             } else {
+                if (yield) sched_yield();
                 got = there();
             }
         }
