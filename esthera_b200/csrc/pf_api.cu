@@ -1018,8 +1018,7 @@ extern "C" pf_status pf_step_submit(pf_filter* f, const pf_step_input* in)
     s = enqueue_step(f, f->d_desc + 2, ir, nullptr, chained);
     if (s != PF_OK) return s;
     f->q_active = 1;
-    f->q_next++;
-    f->steps_done++;
+    f->q_next = f->steps_done = (int32_t)((uint32_t)f->q_next + 1u);
     f->q_pending++;
     return PF_OK;
 }
@@ -1037,8 +1036,8 @@ extern "C" pf_status pf_step_collect(pf_filter* f, pf_estimate* out, int32_t max
     const bool yield = (flags & cudaDeviceScheduleMask) == cudaDeviceScheduleYield ||
                        (flags & cudaDeviceScheduleMask) == cudaDeviceScheduleBlockingSync;
     while (*count < max && f->q_pending > 0) {
-        const int32_t k = f->q_next - f->q_pending;  // oldest pending step
-        const int slot = (int)((uint32_t)k % PF_QUEUE_DEPTH);
+        const uint32_t k = (uint32_t)f->q_next - (uint32_t)f->q_pending;  // oldest pending step
+        const int slot = (int)(k % PF_QUEUE_DEPTH);
         auto there = [&] { return __atomic_load_n(f->h_q_done + slot, __ATOMIC_ACQUIRE) != 0; };
         bool got = there();
         for (unsigned i = 1; !got && (wait || i == 1); ++i) {
@@ -1056,7 +1055,7 @@ extern "C" pf_status pf_step_collect(pf_filter* f, pf_estimate* out, int32_t max
         }
         if (!got) break;
         out[*count] = f->h_q_est[slot];
-        out[(*count)++].step = k + 1;
+        out[(*count)++].step = (int32_t)(k + 1u);
         f->q_pending--;
     }
     return PF_OK;

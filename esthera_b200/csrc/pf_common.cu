@@ -477,7 +477,7 @@ cudaError_t launch_shard_estimate(const FilterDesc& D, int S, const float* best_
 // every kernel of the step that reads it is enqueued before it.
 __global__ void k_counter_add(int32_t* ctr, int32_t n)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *ctr += n;
+    if (threadIdx.x == 0 && blockIdx.x == 0) *ctr = (int32_t)((uint32_t)*ctr + (uint32_t)n);
 }
 
 cudaError_t launch_counter_add(int32_t* ctr, int32_t n, cudaStream_t st)

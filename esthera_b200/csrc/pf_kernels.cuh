@@ -171,12 +171,14 @@ struct InputRef {
 };
 
 // Step number within the run: the device counter, else the host-given number.
-__device__ __forceinline__ int32_t run_step(const InputRef& in) { return in.ctr ? *in.ctr + in.add : in.step; }
+// (Counters add as unsigned numbers: a run past 2^31 steps wraps.)
+__device__ __forceinline__ uint32_t run_counter(const InputRef& in) { return (uint32_t)*in.ctr + (uint32_t)in.add; }
+__device__ __forceinline__ int32_t run_step(const InputRef& in) { return in.ctr ? (int32_t)run_counter(in) : in.step; }
 
 __device__ __forceinline__ int64_t step_index(const InputRef& in)
 {
     // unsigned: a counter that wrapped past 2^31 steps still maps into [0, cap)
-    return in.ctr ? (int64_t)((uint32_t)(*in.ctr + in.add) % (uint32_t)(in.cap > 0 ? in.cap : 1)) : in.slot;
+    return in.ctr ? (int64_t)(run_counter(in) % (uint32_t)(in.cap > 0 ? in.cap : 1)) : in.slot;
 }
 
 // Tells the host that the estimate is written (one lane, after the warp that
@@ -1063,7 +1065,7 @@ __device__ __forceinline__ void estimate_group(const FilterDesc& D, int g, const
     const int lane = threadIdx.x;
     const int b = g << 5, ng = (D.N + 31) >> 5;
     const int NV = 2 + S + D.na;
-    const int32_t step_no = in.ctr ? *in.ctr + in.add + 1 : 0;
+    const int32_t step_no = in.ctr ? (int32_t)(run_counter(in) + 1u) : 0;
     // winners as filter-wide indices (a shard's sub-filters start at b0)
     group_row<S, STAGED>(D, D.part + (int64_t)b * kPartStride, D.winner + b, min(32, D.N - b), NV, b + D.b0, lane,
                          D.gpart + (int64_t)g * kPartStride, smem);
@@ -1088,7 +1090,7 @@ __device__ __forceinline__ void estimate_group(const FilterDesc& D, int g, const
         if (ng > 1) *D.est_ctr = 0;
         publish_estimate(in);
         __threadfence();
-        if (step_ctr) *step_ctr += in.inc;
+        if (step_ctr) *step_ctr = (int32_t)((uint32_t)*step_ctr + (uint32_t)in.inc);
     }
 }
 

@@ -71,14 +71,15 @@ __device__ __forceinline__ void estimate_last_done(const FilterDesc& D, const St
     }
     const int par = (*X.steps) & 1;
     const float* cur_tmp = par ? X.tmp2 : D.tmp;
-    estimate_write<S>(D, lane, ng, NV, gm, bk, bi, cur_tmp, D.est[step_index(in)], in.ctr ? *in.ctr + 1 : 0);
+    estimate_write<S>(D, lane, ng, NV, gm, bk, bi, cur_tmp, D.est[step_index(in)],
+                      in.ctr ? (int32_t)(run_counter(in) + 1u) : 0);
     if (lane == 0) {
         publish_estimate(in);
         *D.est_ctr = 0;
         *X.need_init = 0;
         __threadfence();
         *X.steps += 1;
-        if (step_ctr) *step_ctr += 1;
+        if (step_ctr) *step_ctr = (int32_t)((uint32_t)*step_ctr + (uint32_t)in.inc);
     }
 }
 
