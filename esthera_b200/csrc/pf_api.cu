@@ -1012,7 +1012,6 @@ extern "C" pf_status pf_step_submit(pf_filter* f, const pf_step_input* in)
     InputRef ir = host_input(f, *in);
     ir.slot = slot;
     ir.done = f->h_q_done + slot;
-    ir.done_value = 1;
     __atomic_store_n(f->h_q_done + slot, 0, __ATOMIC_RELEASE);
     f->q_active = 0;  // (until the launches are in the stream)
     s = enqueue_step(f, f->d_desc + 2, ir, nullptr, chained);

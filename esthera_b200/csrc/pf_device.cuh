@@ -350,9 +350,9 @@ struct F2 {
         asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
     }
 };
-// Neither operand may be a product: the assembler fuses a packed multiply with
-// the packed add that takes its result (and with fma2(product, 1, b)) whatever
-// -fmad says.  Subtract instead: fma2(b, -1, product) keeps both roundings.
+// Neither operand may be a product: the sum of a packed product came out with
+// one rounding instead of two (an ulp off the scalar code), with -fmad=false
+// too.  Subtract instead: fma2(b, -1, product) keeps both roundings.
 __device__ __forceinline__ F2 operator+(F2 a, F2 b)
 {
     F2 r;
@@ -806,22 +806,6 @@ __device__ __forceinline__ double scan_f64(const float (&w)[E], double (&cum)[E]
     return red[32 + NW - 1];
 }
 
-// Number of cum[] entries <= x (upper bound), clamped to M-1.
-template <int M>
-__device__ __forceinline__ int upper_count(const double* cum, double x)
-{
-    int lo = 0, hi = M;
-#pragma unroll
-    for (int it = 0; it < 11; ++it) {
-        if (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (cum[mid] <= x) lo = mid + 1;
-            else hi = mid;
-        }
-    }
-    return lo < M ? lo : M - 1;
-}
-
 // First i in [0, M] with (u0 + i) * step >= t, from any start.  A call of its
 // own: rarely taken, and inlined at every boundary it would only make the
 // kernel's code, which a launch fetches from memory, longer.
@@ -842,8 +826,8 @@ static __device__ __noinline__ int first_output(double u0, double step, double t
 // outputs tile [0, M) in ascending order.  A run is marked where it starts and
 // at each warp's first output inside it (mark[], zeroed by the caller before
 // its last barrier), and every output takes the largest mark at or before it
-// within its warp.  pos(i) and the comparisons are those of upper_count(cum,
-// pos(i)), so every output selects the same input (pos is non-decreasing in
+// within its warp.  pos(i) and the comparisons are those of a search of cum[] for
+// pos(i), so every output selects the same input (pos is non-decreasing in
 // i).  Synchronises the CTA.
 //
 // Bound: issue slots.  Measured with the rest of the resampling kernel: 6M

@@ -166,7 +166,6 @@ struct InputRef {
     int32_t inlined = 0;
     int32_t slot = 0;
     int32_t* done = nullptr;
-    int32_t done_value = 0;
     pf_step_input input = {};
 };
 
@@ -187,7 +186,7 @@ __device__ __forceinline__ void publish_estimate(const InputRef& in)
 {
     if (!in.done) return;
     __threadfence_system();
-    *const_cast<volatile int32_t*>(in.done) = in.done_value;
+    *const_cast<volatile int32_t*>(in.done) = 1;
 }
 
 // A status bit (one byte each, so that no atomic is needed on the pinned host

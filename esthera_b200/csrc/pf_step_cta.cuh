@@ -11,9 +11,9 @@
 //      particles, written in place)
 //   G  this step's MTGP32 draws (normals -> shared memory, uniforms -> ru),
 //      Box-Muller
-//   P  propagate + log-likelihood of the thread's E particles
-//   S  bitonic sort; sorted keys and particles -> this step's half; winner;
-//      FP64 estimate partials
+//   P  propagate + log-likelihood of the thread's E particles; FP64 estimate
+//      partials
+//   S  sort; sorted keys and particles -> this step's half; winner
 //   E  group / final estimate by the last CTAs to finish (two-level tickets)
 // The arithmetic of every phase is the split pipeline's (k_exchange_resample
 // + k_sample_sort), so both give bit-identical particles and estimates; the
@@ -146,7 +146,8 @@ __global__ void __launch_bounds__(M / E, pf_min_blocks(M / E, pf_k1_warps(Mdl::S
         },
         [&](int v, const float(&o)[E]) { stv<E>(cur_tmp + v * T + base, o); });
 
-    // ---- E (warp 0 wrote the partials)
+    // ---- E (several warps wrote the partials and warp 0 the winner: the sort's
+    // barriers lie between the partials and warp 0's fence and ticket)
     if (tid < 32) estimate_last_done<S>(D, X, b, in, step_ctr, tid);
 }
 

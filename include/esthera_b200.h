@@ -247,13 +247,16 @@ pf_status pf_step(pf_filter* f, const pf_step_input* in, pf_estimate* out);
 /* Device-resident run: d_inputs[capacity] and d_estimates[capacity] in device
  * memory; resets the step counter and runs `steps` steps (step k reads
  * d_inputs[k % capacity], writes d_estimates[k % capacity]).  Asynchronous on
- * the filter's stream: one step -- and, once the filter has run 64, four and
- * sixteen steps -- is captured into a CUDA graph (once per argument set) and
- * replayed with a device step counter.  pf_synchronize() waits. */
+ * the filter's stream: one step is captured into a CUDA graph (once per
+ * argument set) and replayed with a device step counter; so are four and sixteen
+ * steps once the steps run over these arrays and those a call has still to run
+ * come to 64 (about 0.1 ms each, in that call).  pf_synchronize() waits. */
 pf_status pf_run_device(pf_filter* f, const pf_step_input* d_inputs, pf_estimate* d_estimates,
                         int32_t capacity, int32_t steps);
 /* Replays `steps` more steps of the run set up by pf_run_device (the step
- * counter continues), e.g. to time steps one at a time. */
+ * counter continues, whatever was submitted or stepped in between), e.g. to time
+ * steps one at a time.  PF_ERR_INVALID before any pf_run_device: submitted
+ * steps set up no run. */
 pf_status pf_run_device_continue(pf_filter* f, int32_t steps);
 /* Pipelined host stepping (no counterpart in the reference, whose driver loop
  * copies each step's estimate back before the next step starts,
@@ -267,7 +270,8 @@ pf_status pf_run_device_continue(pf_filter* f, int32_t steps);
  * does a submit after another call stepped the filter while steps are pending.
  * A submit while the filter's stream is being captured is refused (PF_ERR_CUDA).
  * pf_step_collect returns up to `max` estimates in submission order; wait != 0
- * blocks until that many are there (or all pending ones), wait == 0 returns those
+ * waits until that many are there (or all pending ones; it polls, giving the core
+ * away between polls on a device set to yield or block), wait == 0 returns those
  * that are.  One host thread per filter. */
 #define PF_QUEUE_DEPTH 64
 pf_status pf_step_submit(pf_filter* f, const pf_step_input* in);
