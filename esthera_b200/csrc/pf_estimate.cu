@@ -154,7 +154,7 @@ __global__ void k_est_clear(unsigned* ticket)
 // -- and, for states of up to 4 variables, of every state row -- are issued
 // before the maximum is reduced, so a sub-filter costs one round trip to
 // memory, and a lane keeps its own sums only for the variables there are.  2^20
-// particles of 3 variables, 2048 sub-filters of 512: 14.4 us a call, against
+// particles of 3 variables, 2048 sub-filters of 512: 15.3 us a call, against
 // 16.4 us with the rows combined by a second kernel and 63.2 us for one 256-thread
 // CTA per sub-filter with 33 sums per thread whatever S was.
 template <int S, int TW, int V>
