@@ -76,7 +76,7 @@ def test_collect_follows_the_schedule_flag(gpu, tmp_path, flag, yields):
                    "long yields(void) { return __atomic_load_n(&n, __ATOMIC_RELAXED); }\n")
     subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-o", str(lib), str(src)], check=True)
     r = subprocess.run([sys.executable, "-c", YIELD_CHILD, str(flag), str(Path(gpu.__file__).parents[1]), str(lib)],
-                       env=dict(os.environ, LD_PRELOAD=str(lib)), capture_output=True, text=True, timeout=300)
+                       env=dict(os.environ, LD_PRELOAD=str(lib), OPENBLAS_NUM_THREADS="1"), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
     n, step, seen = map(int, r.stdout.split())
     assert (n, step) == (31, 32)
